@@ -6,226 +6,369 @@
 // :1051-1075 (Fermat's little theorem check q < p, checksum mix64(q ^ p * GOLD), symmetric
 // residue A).
 //
-// The device form keeps the same mathematics with a different number layout: N = p^2 is
-// held in K 32-bit limbs (K = 3, R = 2^96, for p < 2^47; K = 4, R = 2^128, for p < 2^63),
-// multiplied with the CIOS Montgomery product on 32x32->64 integer multiply-adds.  The form
-// of 1 (R mod N) is found by doubling 2^(bitlen(N)-1) up to R, exactly; the reference's
-// double-precision quotient estimates are not used.  The exponent p - 1 is processed left
-// to right: square, then double when the bit is 1 (base 2 needs no multiplier table).  Where
-// 8N < R (p < 2^46 with three limbs, p < 2^62 with four) the two are one product,
-// x (x 2^bit) / R, the doubling being a funnel shift of one operand.
+// The device form keeps the same mathematics with a different number layout and exponent: N = p^2
+// is held in K 32-bit limbs (K = 3, R = 2^96, for p < 2^47; K = 4, R = 2^128, for p < 2^63).
+//
+//  * The ladder computes 2^-(p-1), not 2^(p-1): in Montgomery form 2^-c is the plain power of two
+//    2^(32K - c), so the ladder starts from the exponent's top six bits with a shift, and neither
+//    R mod N nor the first six squarings are needed.  2^-(p-1) = 1 + q'p (mod p^2) exactly when
+//    2^(p-1) = 1 + qp, with q = -q' (mod p).
+//  * Five exponent bits at a time: five squarings, then x <- x 2^-c for a digit c = 1 .. 32, which
+//    is a shift left by 32 - c and one word of Montgomery reduction.  Digits 1 .. 32 instead of
+//    0 .. 31 are reached by taking 1 from every digit position beforehand (p - 1 - off).
+//  * Values stay in [0, 2^(32K-1)) without a comparison: x -> (x^2 + mN) / R < x^2 / R + N, and
+//    both terms are below 2^(32K-2).  Leaving Montgomery form gives the residue in [0, N].
+//  * What bounds it is the multiply pipe.  Measured on B200, clocks of an SM per warp instruction:
+//    32-bit low product 0.51, high product 1.0, 64-bit product with or without accumulation and
+//    carry 1.02, an add with carry about 0.4.  So a product of two limbs is one 64-bit
+//    multiply-add (mad.lo.cc directly followed by madc.hi.cc), and a squaring forms each cross
+//    product once: 18 products at K = 3, a floor of 16.8 clocks; this form takes 17.8 (K = 4:
+//    35.2 against a floor of 28.5).  Low and high halves in separate carry chains took 57
+//    low-product units (29 clocks).  Sums at even and odd limb positions are kept apart until the
+//    end: the pair of registers a 64-bit product lands in is aligned, and sharing one set of sums
+//    between even and odd positions cost moves (23.3 clocks at K = 3, 43.4 at K = 4).
 #include "mp_common.cuh"
 
-// t[0..K] += a[0..K-1] * b: the low halves of the products in one carry chain, then the high
-// halves one word up in a second; each chain is one asm block, so that nothing between its
-// instructions can touch the carry flag.  The multiply-adds run on the multiply pipe.  The
-// callers keep t below 2^(32 (K + 1)), so nothing carries out of t[K] (see mmul_lazy).
+// x <- x^2 / R (mod N): see the header for the bounds; np = -N^-1 mod 2^32
 template <int K>
-__device__ __forceinline__ void mac_row(u32 (&t)[K + 1], const u32 (&a)[K], u32 b);
+__device__ __forceinline__ void msqr(u32 (&x)[K], const u32 (&n)[K], u32 np);
+
+// a0 .. hold the sums at even limb positions, b1 .. those at odd ones; a word of reduction adds m N
+// with m = (lowest word) np, and the word it does not clear joins the other set.  Products that
+// start a pair of sums take the carry below them (their sum cannot overflow).
+template <>
+__device__ __forceinline__ void msqr<3>(u32 (&x)[3], const u32 (&n)[3], u32 np)
+{
+    asm("{\n\t.reg .u32 a0, a1, a2, a3, a4, a5, b1, b2, b3, b4, b5, e1, e2, f2, m;\n\t"
+        "shl.b32         e1, %1, 1;\n\t"                   // 2 (x1, x2) = (e1, e2), 2 x2 = f2
+        "shf.l.wrap.b32  e2, %1, %2, 1;\n\t"
+        "shl.b32         f2, %2, 1;\n\t"
+        "mul.lo.u32      a0, %0, %0;\n\t"
+        "mul.hi.u32      a1, %0, %0;\n\t"
+        "mul.lo.u32      a2, %1, %1;\n\t"
+        "mul.hi.u32      a3, %1, %1;\n\t"
+        "mad.lo.cc.u32   a2, %0, e2, a2;\n\t"
+        "madc.hi.cc.u32  a3, %0, e2, a3;\n\t"
+        "madc.lo.cc.u32  a4, %2, %2, 0;\n\t"
+        "madc.hi.u32     a5, %2, %2, 0;\n\t"
+        "mul.lo.u32      b1, %0, e1;\n\t"
+        "mul.hi.u32      b2, %0, e1;\n\t"
+        "mul.lo.u32      m, a0, %6;\n\t"                   // word 0
+        "mad.lo.cc.u32   b1, m, %4, b1;\n\t"
+        "madc.hi.cc.u32  b2, m, %4, b2;\n\t"
+        "madc.lo.cc.u32  b3, %1, f2, 0;\n\t"
+        "madc.hi.u32     b4, %1, f2, 0;\n\t"
+        "mad.lo.cc.u32   a0, m, %3, a0;\n\t"
+        "madc.hi.cc.u32  a1, m, %3, a1;\n\t"
+        "madc.lo.cc.u32  a2, m, %5, a2;\n\t"
+        "madc.hi.cc.u32  a3, m, %5, a3;\n\t"
+        "addc.cc.u32     a4, a4, 0;\n\t"
+        "addc.u32        a5, a5, 0;\n\t"
+        "add.cc.u32      b1, b1, a1;\n\t"                  // word 1
+        "mul.lo.u32      m, b1, %6;\n\t"
+        "madc.lo.cc.u32  a2, m, %4, a2;\n\t"
+        "madc.hi.cc.u32  a3, m, %4, a3;\n\t"
+        "addc.cc.u32     a4, a4, 0;\n\t"
+        "addc.u32        a5, a5, 0;\n\t"
+        "mad.lo.cc.u32   b1, m, %3, b1;\n\t"
+        "madc.hi.cc.u32  b2, m, %3, b2;\n\t"
+        "madc.lo.cc.u32  b3, m, %5, b3;\n\t"
+        "madc.hi.cc.u32  b4, m, %5, b4;\n\t"
+        "addc.u32        b5, 0, 0;\n\t"
+        "add.cc.u32      a2, a2, b2;\n\t"                  // word 2
+        "mul.lo.u32      m, a2, %6;\n\t"
+        "madc.lo.cc.u32  b3, m, %4, b3;\n\t"
+        "madc.hi.cc.u32  b4, m, %4, b4;\n\t"
+        "addc.u32        b5, b5, 0;\n\t"
+        "mad.lo.cc.u32   a2, m, %3, a2;\n\t"
+        "madc.hi.cc.u32  a3, m, %3, a3;\n\t"
+        "madc.lo.cc.u32  a4, m, %5, a4;\n\t"
+        "madc.hi.u32     a5, m, %5, a5;\n\t"
+        "add.cc.u32      %0, a3, b3;\n\t"
+        "addc.cc.u32     %1, a4, b4;\n\t"
+        "addc.u32        %2, a5, b5;\n\t}"
+        : "+r"(x[0]), "+r"(x[1]), "+r"(x[2])
+        : "r"(n[0]), "r"(n[1]), "r"(n[2]), "r"(np));
+}
 
 template <>
-__device__ __forceinline__ void mac_row<3>(u32 (&t)[4], const u32 (&a)[3], u32 b)
+__device__ __forceinline__ void msqr<4>(u32 (&x)[4], const u32 (&n)[4], u32 np)
 {
-    asm("mad.lo.cc.u32  %0, %4, %7, %0;\n\t"
-        "madc.lo.cc.u32 %1, %5, %7, %1;\n\t"
-        "madc.lo.cc.u32 %2, %6, %7, %2;\n\t"
-        "addc.u32       %3, %3, 0;\n\t"
-        "mad.hi.cc.u32  %1, %4, %7, %1;\n\t"
-        "madc.hi.cc.u32 %2, %5, %7, %2;\n\t"
-        "madc.hi.u32    %3, %6, %7, %3;"
-        : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(b));
+    asm("{\n\t.reg .u32 a0, a1, a2, a3, a4, a5, a6, a7, b1, b2, b3, b4, b5, b6, b7, e1, e2, e3, f2, g3, m;\n\t"
+        "shl.b32         e1, %1, 1;\n\t"                   // 2 (x1, x2, x3) = (e1, e2, e3),
+        "shf.l.wrap.b32  e2, %1, %2, 1;\n\t"               // 2 (x2, x3) = (f2, e3), 2 x3 = g3
+        "shf.l.wrap.b32  e3, %2, %3, 1;\n\t"
+        "shl.b32         f2, %2, 1;\n\t"
+        "shl.b32         g3, %3, 1;\n\t"
+        "mul.lo.u32      a0, %0, %0;\n\t"
+        "mul.hi.u32      a1, %0, %0;\n\t"
+        "mul.lo.u32      a2, %1, %1;\n\t"
+        "mul.hi.u32      a3, %1, %1;\n\t"
+        "mad.lo.cc.u32   a2, %0, e2, a2;\n\t"
+        "madc.hi.cc.u32  a3, %0, e2, a3;\n\t"
+        "madc.lo.cc.u32  a4, %2, %2, 0;\n\t"
+        "madc.hi.u32     a5, %2, %2, 0;\n\t"
+        "mul.lo.u32      b1, %0, e1;\n\t"
+        "mul.hi.u32      b2, %0, e1;\n\t"
+        "mul.lo.u32      b3, %0, e3;\n\t"
+        "mul.hi.u32      b4, %0, e3;\n\t"
+        "mul.lo.u32      m, a0, %8;\n\t"                   // word 0
+        "mad.lo.cc.u32   b1, m, %5, b1;\n\t"
+        "madc.hi.cc.u32  b2, m, %5, b2;\n\t"
+        "madc.lo.cc.u32  b3, m, %7, b3;\n\t"
+        "madc.hi.cc.u32  b4, m, %7, b4;\n\t"
+        "madc.lo.cc.u32  b5, %2, g3, 0;\n\t"
+        "madc.hi.u32     b6, %2, g3, 0;\n\t"
+        "mad.lo.cc.u32   b3, %1, f2, b3;\n\t"
+        "madc.hi.cc.u32  b4, %1, f2, b4;\n\t"
+        "addc.cc.u32     b5, b5, 0;\n\t"
+        "addc.u32        b6, b6, 0;\n\t"
+        "mad.lo.cc.u32   a0, m, %4, a0;\n\t"
+        "madc.hi.cc.u32  a1, m, %4, a1;\n\t"
+        "madc.lo.cc.u32  a2, m, %6, a2;\n\t"
+        "madc.hi.cc.u32  a3, m, %6, a3;\n\t"
+        "madc.lo.cc.u32  a4, %1, e3, a4;\n\t"
+        "madc.hi.cc.u32  a5, %1, e3, a5;\n\t"
+        "madc.lo.cc.u32  a6, %3, %3, 0;\n\t"
+        "madc.hi.u32     a7, %3, %3, 0;\n\t"
+        "add.cc.u32      b1, b1, a1;\n\t"                  // word 1
+        "mul.lo.u32      m, b1, %8;\n\t"
+        "madc.lo.cc.u32  a2, m, %5, a2;\n\t"
+        "madc.hi.cc.u32  a3, m, %5, a3;\n\t"
+        "madc.lo.cc.u32  a4, m, %7, a4;\n\t"
+        "madc.hi.cc.u32  a5, m, %7, a5;\n\t"
+        "addc.cc.u32     a6, a6, 0;\n\t"
+        "addc.u32        a7, a7, 0;\n\t"
+        "mad.lo.cc.u32   b1, m, %4, b1;\n\t"
+        "madc.hi.cc.u32  b2, m, %4, b2;\n\t"
+        "madc.lo.cc.u32  b3, m, %6, b3;\n\t"
+        "madc.hi.cc.u32  b4, m, %6, b4;\n\t"
+        "addc.cc.u32     b5, b5, 0;\n\t"
+        "addc.cc.u32     b6, b6, 0;\n\t"
+        "addc.u32        b7, 0, 0;\n\t"
+        "add.cc.u32      a2, a2, b2;\n\t"                  // word 2
+        "mul.lo.u32      m, a2, %8;\n\t"
+        "madc.lo.cc.u32  b3, m, %5, b3;\n\t"
+        "madc.hi.cc.u32  b4, m, %5, b4;\n\t"
+        "madc.lo.cc.u32  b5, m, %7, b5;\n\t"
+        "madc.hi.cc.u32  b6, m, %7, b6;\n\t"
+        "addc.u32        b7, b7, 0;\n\t"
+        "mad.lo.cc.u32   a2, m, %4, a2;\n\t"
+        "madc.hi.cc.u32  a3, m, %4, a3;\n\t"
+        "madc.lo.cc.u32  a4, m, %6, a4;\n\t"
+        "madc.hi.cc.u32  a5, m, %6, a5;\n\t"
+        "addc.cc.u32     a6, a6, 0;\n\t"
+        "addc.u32        a7, a7, 0;\n\t"
+        "add.cc.u32      b3, b3, a3;\n\t"                  // word 3
+        "mul.lo.u32      m, b3, %8;\n\t"
+        "madc.lo.cc.u32  a4, m, %5, a4;\n\t"
+        "madc.hi.cc.u32  a5, m, %5, a5;\n\t"
+        "madc.lo.cc.u32  a6, m, %7, a6;\n\t"
+        "madc.hi.u32     a7, m, %7, a7;\n\t"
+        "mad.lo.cc.u32   b3, m, %4, b3;\n\t"
+        "madc.hi.cc.u32  b4, m, %4, b4;\n\t"
+        "madc.lo.cc.u32  b5, m, %6, b5;\n\t"
+        "madc.hi.cc.u32  b6, m, %6, b6;\n\t"
+        "addc.u32        b7, b7, 0;\n\t"
+        "add.cc.u32      %0, a4, b4;\n\t"
+        "addc.cc.u32     %1, a5, b5;\n\t"
+        "addc.cc.u32     %2, a6, b6;\n\t"
+        "addc.u32        %3, a7, b7;\n\t}"
+        : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3])
+        : "r"(n[0]), "r"(n[1]), "r"(n[2]), "r"(n[3]), "r"(np));
+}
+
+// x <- (x 2^sh + m N) / 2^32 (mod N), sh in [0, 31]: below x / 2 + N
+template <int K>
+__device__ __forceinline__ void mshift(u32 (&x)[K], u32 sh, const u32 (&n)[K], u32 np);
+
+template <>
+__device__ __forceinline__ void mshift<3>(u32 (&x)[3], u32 sh, const u32 (&n)[3], u32 np)
+{
+    asm("{\n\t.reg .u32 t0, t1, t2, t3, b1, b2, m;\n\t"
+        "shl.b32         t0, %0, %7;\n\t"
+        "shf.l.wrap.b32  t1, %0, %1, %7;\n\t"
+        "shf.l.wrap.b32  t2, %1, %2, %7;\n\t"
+        "shf.l.wrap.b32  t3, %2, 0, %7;\n\t"
+        "mul.lo.u32      m, t0, %6;\n\t"
+        "mul.lo.u32      b1, m, %4;\n\t"
+        "mul.hi.u32      b2, m, %4;\n\t"
+        "mad.lo.cc.u32   t0, m, %3, t0;\n\t"
+        "madc.hi.cc.u32  t1, m, %3, t1;\n\t"
+        "madc.lo.cc.u32  t2, m, %5, t2;\n\t"
+        "madc.hi.u32     t3, m, %5, t3;\n\t"
+        "add.cc.u32      %0, t1, b1;\n\t"
+        "addc.cc.u32     %1, t2, b2;\n\t"
+        "addc.u32        %2, t3, 0;\n\t}"
+        : "+r"(x[0]), "+r"(x[1]), "+r"(x[2])
+        : "r"(n[0]), "r"(n[1]), "r"(n[2]), "r"(np), "r"(sh));
 }
 
 template <>
-__device__ __forceinline__ void mac_row<4>(u32 (&t)[5], const u32 (&a)[4], u32 b)
+__device__ __forceinline__ void mshift<4>(u32 (&x)[4], u32 sh, const u32 (&n)[4], u32 np)
 {
-    asm("mad.lo.cc.u32  %0, %5, %9, %0;\n\t"
-        "madc.lo.cc.u32 %1, %6, %9, %1;\n\t"
-        "madc.lo.cc.u32 %2, %7, %9, %2;\n\t"
-        "madc.lo.cc.u32 %3, %8, %9, %3;\n\t"
-        "addc.u32       %4, %4, 0;\n\t"
-        "mad.hi.cc.u32  %1, %5, %9, %1;\n\t"
-        "madc.hi.cc.u32 %2, %6, %9, %2;\n\t"
-        "madc.hi.cc.u32 %3, %7, %9, %3;\n\t"
-        "madc.hi.u32    %4, %8, %9, %4;"
-        : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b));
+    asm("{\n\t.reg .u32 t0, t1, t2, t3, t4, b1, b2, b3, b4, m;\n\t"
+        "shl.b32         t0, %0, %9;\n\t"
+        "shf.l.wrap.b32  t1, %0, %1, %9;\n\t"
+        "shf.l.wrap.b32  t2, %1, %2, %9;\n\t"
+        "shf.l.wrap.b32  t3, %2, %3, %9;\n\t"
+        "shf.l.wrap.b32  t4, %3, 0, %9;\n\t"
+        "mul.lo.u32      m, t0, %8;\n\t"
+        "mul.lo.u32      b1, m, %5;\n\t"
+        "mul.hi.u32      b2, m, %5;\n\t"
+        "mul.lo.u32      b3, m, %7;\n\t"
+        "mul.hi.u32      b4, m, %7;\n\t"
+        "mad.lo.cc.u32   t0, m, %4, t0;\n\t"
+        "madc.hi.cc.u32  t1, m, %4, t1;\n\t"
+        "madc.lo.cc.u32  t2, m, %6, t2;\n\t"
+        "madc.hi.cc.u32  t3, m, %6, t3;\n\t"
+        "addc.u32        t4, t4, 0;\n\t"
+        "add.cc.u32      %0, t1, b1;\n\t"
+        "addc.cc.u32     %1, t2, b2;\n\t"
+        "addc.cc.u32     %2, t3, b3;\n\t"
+        "addc.u32        %3, t4, b4;\n\t}"
+        : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3])
+        : "r"(n[0]), "r"(n[1]), "r"(n[2]), "r"(n[3]), "r"(np), "r"(sh));
 }
 
-// t - n with the borrow out in one chain: returns 0 when t >= n, all ones otherwise
+// leave Montgomery form: K words of reduction bring x / R into [0, N]
 template <int K>
-__device__ __forceinline__ u32 sub_n(u32 (&d)[K], const u32 (&t)[K], const u32 (&n)[K]);
-
-template <>
-__device__ __forceinline__ u32 sub_n<3>(u32 (&d)[3], const u32 (&t)[3], const u32 (&n)[3])
+__device__ __forceinline__ void mleave(u32 (&x)[K], const u32 (&n)[K], u32 np)
 {
-    u32 bw;
-    asm("sub.cc.u32  %0, %4, %7;\n\t"
-        "subc.cc.u32 %1, %5, %8;\n\t"
-        "subc.cc.u32 %2, %6, %9;\n\t"
-        "subc.u32    %3, 0, 0;"
-        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(bw)
-        : "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(n[0]), "r"(n[1]), "r"(n[2]));
-    return bw;
-}
-
-template <>
-__device__ __forceinline__ u32 sub_n<4>(u32 (&d)[4], const u32 (&t)[4], const u32 (&n)[4])
-{
-    u32 bw;
-    asm("sub.cc.u32  %0, %5, %9;\n\t"
-        "subc.cc.u32 %1, %6, %10;\n\t"
-        "subc.cc.u32 %2, %7, %11;\n\t"
-        "subc.cc.u32 %3, %8, %12;\n\t"
-        "subc.u32    %4, 0, 0;"
-        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(bw)
-        : "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]), "r"(n[0]), "r"(n[1]), "r"(n[2]), "r"(n[3]));
-    return bw;
-}
-
-template <int K>
-__device__ __forceinline__ void cond_sub(u32 (&t)[K], u32 top, const u32 (&n)[K])
-{
-    // t (with carry word `top`) < 2N: subtract N once if t >= N
-    u32 d[K];
-    const u32 bw = sub_n<K>(d, t, n);
-    const bool ge = top || !bw;
-#pragma unroll
-    for (int j = 0; j < K; j++) t[j] = ge ? d[j] : t[j];
-}
-
-// r = a * b / R mod N, CIOS with 32-bit limbs: per word b[i], t += a b[i], then t += m N with
-// m = t[0] (-N^-1) mod 2^32, which clears t[0], and t shifts down a word.  With a, b < 2N and
-// 4N < R the result (ab + mN) / R is below N (4N / R + 1) < 2N, so values stay in [0, 2N)
-// without a subtraction (lazy reduction); only the value that leaves the loop is reduced.
-// Bounds: before a row pair t < 3N (K words), after it t < 3N (1 + 2^32) < 2^(32 (K + 1)).
-template <int K>
-__device__ __forceinline__ void mmul_lazy(u32 (&r)[K], const u32 (&a)[K], const u32 (&b)[K], const u32 (&n)[K],
-                                          u32 np)
-{
-    u32 t[K + 1];
-#pragma unroll
-    for (int j = 0; j < K + 1; j++) t[j] = 0;
 #pragma unroll
     for (int i = 0; i < K; i++) {
-        mac_row<K>(t, a, b[i]);
-        const u32 m = t[0] * np;
-        mac_row<K>(t, n, m);
+        const u32 m = x[0] * np;
+        u64 c = (u64)m * n[0] + x[0];
 #pragma unroll
-        for (int j = 0; j < K; j++) t[j] = t[j + 1];
-        t[K] = 0;
+        for (int j = 1; j < K; j++) {
+            c = (u64)m * n[j] + x[j] + (c >> 32);
+            x[j - 1] = (u32)c;
+        }
+        x[K - 1] = (u32)(c >> 32);
     }
-#pragma unroll
-    for (int j = 0; j < K; j++) r[j] = t[j];
 }
 
-// the same, reduced to [0, N) (for a product below 2N)
+// N = p^2, -N^-1 mod 2^32 and p^-1 mod 2^64
 template <int K>
-__device__ __forceinline__ void mmul(u32 (&r)[K], const u32 (&a)[K], const u32 (&b)[K], const u32 (&n)[K], u32 np)
+__device__ __forceinline__ void fermat_modulus(u64 p, u32 (&n)[K], u32 &np, u64 &pinv)
 {
-    mmul_lazy<K>(r, a, b, n, np);
-    cond_sub<K>(r, 0u, n);
-}
-
-// x = 2x, reduced below m (x < m, 2m <= R): m = N keeps [0, N), m = 2N keeps [0, 2N)
-template <int K>
-__device__ __forceinline__ void mdbl(u32 (&x)[K], const u32 (&n)[K])
-{
-    u32 y[K];
-    y[0] = x[0] << 1;
-#pragma unroll
-    for (int j = 1; j < K; j++) y[j] = (x[j] << 1) | (x[j - 1] >> 31);
-    cond_sub<K>(y, 0u, n);
-#pragma unroll
-    for (int j = 0; j < K; j++) x[j] = y[j];
+    pinv = (3 * p) ^ 2;
+    pinv *= 2 - p * pinv;
+    pinv *= 2 - p * pinv;
+    pinv *= 2 - p * pinv;
+    pinv *= 2 - p * pinv;
+    np = 0u - (u32)(pinv * pinv);
+    const u64 N0 = p * p, N1 = __umul64hi(p, p);
+    n[0] = (u32)N0; n[1] = (u32)(N0 >> 32); n[2] = (u32)N1;
+    if (K == 4) n[K - 1] = (u32)(N1 >> 32);
 }
 
 struct FermOut { u64 q; bool ok; };
 
-// q_p(2) for odd p >= 3 (p < 2^47 for K = 3, p < 2^63 for K = 4)
+// the quotient's definition, q = (r - 1) p^-1 mod 2^64 and q < p with r = 2^(p-1) mod N, for a p
+// that is no prime and has 2^(p-1) <> 1 (mod p): r itself, by squaring and doubling from R mod N
+template <int K>
+__device__ __forceinline__ u64 fermat_not_one(u64 p)
+{
+    u32 n[K], x[K], np;
+    u64 pinv;
+    fermat_modulus<K>(p, n, np, pinv);
+    const auto less_n = [&](u32 (&t)[K]) {             // t - N if t >= N
+        u32 d[K];
+        u64 b = 0;
+        for (int j = 0; j < K; j++) {
+            b = (u64)t[j] - n[j] - b;
+            d[j] = (u32)b;
+            b = (b >> 32) & 1;
+        }
+        for (int j = 0; j < K; j++) t[j] = b ? t[j] : d[j];
+    };
+    const auto twice = [&](u32 (&t)[K]) {              // t < N, 2N < R
+        for (int j = K - 1; j > 0; j--) t[j] = __funnelshift_l(t[j - 1], t[j], 1);
+        t[0] <<= 1;
+        less_n(t);
+    };
+    for (int j = 0; j < K; j++) x[j] = j == 0;
+    for (int i = 0; i < 32 * K; i++) twice(x);
+    const u64 e = p - 1;
+    for (int b = 63 - __clzll((long long)e); b >= 0; b--) {
+        msqr<K>(x, n, np);                             // below N^2 / R + N < 2N
+        less_n(x);
+        if ((e >> b) & 1) twice(x);
+    }
+    mleave<K>(x, n, np);
+    less_n(x);
+    const u64 q = (((u64)x[0] | ((u64)x[1] << 32)) - 1) * pinv;
+    return q < p ? q : ~0ull;
+}
+
+// q_p(2) for odd p >= 3 (p < 2^47 for K = 3, p < 2^63 for K = 4); ok is false when 2^(p-1) <> 1
+// (mod p), which happens for no prime
 template <int K>
 __device__ __forceinline__ FermOut fermat_one(u64 p)
 {
-    u64 pinv = (3 * p) ^ 2;
-    pinv *= 2 - p * pinv;
-    pinv *= 2 - p * pinv;
-    pinv *= 2 - p * pinv;
-    pinv *= 2 - p * pinv;
-    const u32 np = 0u - (u32)(pinv * pinv);            // -N^-1 mod 2^32
-    const u64 N0 = p * p, N1 = __umul64hi(p, p);
-    u32 n[K];
-    n[0] = (u32)N0; n[1] = (u32)(N0 >> 32); n[2] = (u32)N1;
-    if (K == 4) n[K - 1] = (u32)(N1 >> 32);
-    // one = R mod N: start at 2^(top bit of N), double up to 2^(32K)
-    const int topbit = N1 ? 64 + 63 - __clzll((long long)N1) : 63 - __clzll((long long)N0);
-    u32 x[K];
-#pragma unroll
-    for (int j = 0; j < K; j++) x[j] = (topbit >> 5) == j ? (1u << (topbit & 31)) : 0u;
-    for (int i = topbit; i < 32 * K; i++) mdbl<K>(x, n);
-    // left-to-right binary exponentiation of 2 to e = p - 1 on representatives in [0, 2N)
-    // (lazy reduction; 4N < R for both limb counts); leading zero bits keep x = 1
-    u32 n2[K];
-    n2[0] = n[0] << 1;
-#pragma unroll
-    for (int j = 1; j < K; j++) n2[j] = (n[j] << 1) | (n[j - 1] >> 31);
+    u32 n[K], np;
+    u64 pinv;
+    fermat_modulus<K>(p, n, np, pinv);
+    // T squarings after the top six bits; w whole digits of five bits below a digit of rem bits
     const u64 e = p - 1;
-    if (p < (K == 3 ? (1ull << 46) : (1ull << 62))) {
-        // 8N < R: the doubling for a 1 bit goes into the product.  x (x 2^bit) / R with
-        // x < 2N and x 2^bit < 4N (a funnel shift, no subtraction) is below
-        // (8N^2 + R N) / R < 2N, so the square-and-double of one bit is one product
-        for (int b = 63 - __clzll((long long)e); b >= 0; b--) {
-            const u32 bit = (u32)(e >> b) & 1u;
-            u32 y[K];
-            y[0] = x[0] << bit;
+    const int L = 64 - __clzll((long long)e), T = L > 6 ? L - 6 : 0;
+    int w = T / 5;
+    const int rem = T - 5 * w;
+    const u64 ones = 0x1084210842108421ull;            // one in every five-bit digit
+    const u64 d = e - ((ones & ((1ull << (5 * w)) - 1)) + (rem ? 1ull << (5 * w) : 0));
+    u32 x[K];
+    const u32 s0 = 32 * K - (u32)(d >> T);             // 2^-c R, c = the top (30 .. 63, or e itself)
 #pragma unroll
-            for (int j = 1; j < K; j++) y[j] = __funnelshift_l(x[j - 1], x[j], bit);
-            mmul_lazy<K>(x, x, y, n, np);
-        }
-    } else {
-        for (int b = 63 - __clzll((long long)e); b >= 0; b--) {
-            mmul_lazy<K>(x, x, x, n, np);
-            u32 y[K];
-#pragma unroll
-            for (int j = 0; j < K; j++) y[j] = x[j];
-            mdbl<K>(y, n2);
-            const bool bit = (e >> b) & 1;
-#pragma unroll
-            for (int j = 0; j < K; j++) x[j] = bit ? y[j] : x[j];
-        }
+    for (int j = 0; j < K; j++) x[j] = (s0 >> 5) == (u32)j ? 1u << (s0 & 31) : 0u;
+    if (rem) {
+        for (int i = 0; i < rem; i++) msqr<K>(x, n, np);
+        mshift<K>(x, 31u - ((u32)(d >> (5 * w)) & ((1u << rem) - 1u)), n, np);
     }
-    // leave Montgomery form: multiply by 1; with x < 2N the product (x + mN) / R is at most N,
-    // and mmul's subtraction brings it to [0, N)
-    u32 one[K];
+    while (--w >= 0) {
 #pragma unroll
-    for (int j = 0; j < K; j++) one[j] = j == 0 ? 1u : 0u;
-    mmul<K>(x, x, one, n, np);
+        for (int i = 0; i < 5; i++) msqr<K>(x, n, np);
+        mshift<K>(x, 31u - ((u32)(d >> (5 * w)) & 31u), n, np);
+    }
+    mleave<K>(x, n, np);
     const u64 r = (u64)x[0] | ((u64)x[1] << 32);
+    const u64 q = (r - 1) * pinv;                      // q' with 2^-(p-1) = 1 + q'p
     FermOut o;
-    o.q = (r - 1) * pinv;
-    o.ok = o.q < p;
+    // 2^-(p-1) = 1 (mod p), so that 1 + q'p is the whole residue, for every prime p
+    const u64 hi = __umul64hi(q, p) + (q * p == ~0ull);
+    const u64 rhi = K == 4 ? (u64)x[2] | ((u64)x[K - 1] << 32) : (u64)x[2];
+    o.ok = q < p && hi == rhi;
+    o.q = q ? p - q : 0;
     return o;
 }
 
-// one prime per thread (ILP = 1) or two interleaved primes per thread (ILP = 2)
+// one prime per thread (ILP = 1) or two interleaved primes per thread (ILP = 2).  The entries that
+// are not ok are done again at the end, from the definition: inside the loop that code cost the
+// ladder registers (5% of the kernel), and no prime needs it
 template <int K, int ILP>
-__global__ void __launch_bounds__(256) fermat_kernel(const u64 *__restrict__ P, u64 count, u64 *__restrict__ Q)
+__global__ void __launch_bounds__(256) fermat_kernel(const u64 *__restrict__ P, u64 count, u64 *Q)
 {
-    const u64 stride = (u64)gridDim.x * blockDim.x * ILP;
-    for (u64 i = ((u64)blockIdx.x * blockDim.x + threadIdx.x) * ILP; i < count; i += stride) {
-        if (ILP == 1) {
-            const u64 p = __ldg(P + i);
-            u64 q = 0;
-            if (p >= 3 && (p & 1)) { const FermOut o = fermat_one<K>(p); q = o.ok ? o.q : ~0ull; }
-            Q[i] = q;
-        } else {
-            const u64 p0 = __ldg(P + i), p1 = i + 1 < count ? __ldg(P + i + 1) : 3;
-            const bool v0 = p0 >= 3 && (p0 & 1), v1 = p1 >= 3 && (p1 & 1);
-            const FermOut o0 = fermat_one<K>(v0 ? p0 : 3), o1 = fermat_one<K>(v1 ? p1 : 3);
-            Q[i] = v0 ? (o0.ok ? o0.q : ~0ull) : 0;
-            if (i + 1 < count) Q[i + 1] = v1 ? (o1.ok ? o1.q : ~0ull) : 0;
+    const u64 stride = (u64)gridDim.x * blockDim.x * ILP, first = ((u64)blockIdx.x * blockDim.x + threadIdx.x) * ILP;
+    bool again = false;
+    for (u64 i = first; i < count; i += stride) {
+        u64 p[ILP];
+        FermOut o[ILP];
+#pragma unroll
+        for (int v = 0; v < ILP; v++) {
+            p[v] = i + v < count ? __ldg(P + i + v) : 0;
+            o[v] = fermat_one<K>(p[v] >= 3 && (p[v] & 1) ? p[v] : 3);
+        }
+#pragma unroll
+        for (int v = 0; v < ILP; v++) {
+            const bool odd = p[v] >= 3 && (p[v] & 1);
+            if (i + v < count) Q[i + v] = odd ? (o[v].ok ? o[v].q : ~0ull) : 0;
+            again |= odd && !o[v].ok;
         }
     }
+    if (!again) return;
+    for (u64 i = first; i < count; i += stride)
+        for (int v = 0; v < ILP; v++)
+            if (i + v < count && Q[i + v] == ~0ull) Q[i + v] = fermat_not_one<K>(__ldg(P + i + v));
 }
 
 // ---- statistics: checksum, near count, FLT errors, hits, ordered hash ----
