@@ -367,15 +367,13 @@ int mp_wieferich_range(mp_handle *h, uint64_t lo, uint64_t hi, mp_wief_stats *ou
     u64 n = 0;
     MP_TRY(mp_sieve_emit_primes(h, lo, hi, nullptr, 0, &n, st));
     MP_CUDA(h, h->ferm_p.ensure((size_t)n * 8 + 8));
-    MP_CUDA(h, h->ferm_q.ensure((size_t)n * 8 + 8));
     MP_CUDA(h, h->stats_out.ensure(sizeof(mp_wief_stats) + 256));
     u64 n2 = 0;
     MP_TRY(mp_sieve_emit_primes(h, lo, hi, h->ferm_p.as<u64>(), n, &n2, st));
     const int variant = ((hi - 1) >> 47 ? 1 : 0) | (h->tune.fermat_variant & 2);
     mp_wief_stats *ds = h->stats_out.as<mp_wief_stats>();
     MP_CUDA(h, cudaEventRecord(h->ev0, st));
-    MP_TRY(mp_fermat_run(h, h->ferm_p.as<u64>(), n, h->ferm_q.as<u64>(), st, variant, nullptr));
-    MP_TRY(mp_fermat_reduce(h, h->ferm_p.as<u64>(), h->ferm_q.as<u64>(), n, ds, st));
+    MP_TRY(mp_fermat_stats(h, h->ferm_p.as<u64>(), n, ds, st, variant));
     MP_CUDA(h, cudaEventRecord(h->ev1, st));
     MP_CUDA(h, cudaMemcpyAsync(out, ds, sizeof *out, cudaMemcpyDeviceToHost, st));
     MP_CUDA(h, cudaStreamSynchronize(st));

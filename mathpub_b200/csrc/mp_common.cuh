@@ -312,7 +312,6 @@ int mp_bpsw_run(mp_handle *h, const u64 *d_n, const u64 *offs, const u32 *lens, 
 const char *mp_bpsw_variant_name(int v);
 int mp_fermat_run(mp_handle *h, const u64 *d_p, u64 count, u64 *d_q, cudaStream_t st,
                   int variant, u64 *d_partials);                     // mp_fermat.cu
-int mp_fermat_reduce(mp_handle *h, const u64 *d_p, const u64 *d_q, u64 count,
-                     mp_wief_stats *d_stats, cudaStream_t st);
+int mp_fermat_stats(mp_handle *h, const u64 *d_p, u64 count, mp_wief_stats *d_stats, cudaStream_t st, int variant);
 void mp_graphs_free(mp_handle *h);                                   // mp_api.cu
 void mp_chain_free(mp_handle *h);                                    // mp_chain.cu
