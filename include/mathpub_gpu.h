@@ -236,9 +236,9 @@ int mp_bpsw_batches(mp_handle *h, const uint64_t *const *lists, const uint32_t *
 
 /* device form: candidates laid out as nlists lists, list i at d_n + offs[i] (offs[i] a
    multiple of 32, host array offs[0..nlists]), verdict words (u32, bit i & 31 of word
-   i >> 5) at d_bits + offs[i] / 32; mode MP_MODE_BATCHED (one persistent launch over
-   every list for trial division and the base-2 test, then two launches for the Lucas test
-   on the base-2 passers) or MP_MODE_PLAIN (one launch per list) */
+   i >> 5) at d_bits + offs[i] / 32; mode MP_MODE_BATCHED (launches over every list at
+   once: trial division, the base-2 test on the survivors, Selfridge's search and the Lucas
+   test on the passers; one launch for a few thousand candidates) or MP_MODE_PLAIN (one launch per list) */
 int mp_bpsw_lists_dev(mp_handle *h, const uint64_t *d_n, const uint64_t *offs,
                       const uint32_t *lens, uint32_t nlists, uint32_t *d_bits, uint32_t mode,
                       void *stream);
@@ -304,7 +304,7 @@ int mp_autotune(mp_handle *h, uint64_t lo, char *report, size_t cap);
  *   MP_TUNE_NO_PIPELINE    1: batched sieve calls as a host loop of wave launches, 0: one
  *                          persistent pipeline launch (with the binned scatter only; the
  *                          staged scatter always runs the wave loop)
- *   MP_TUNE_BPSW_VARIANT   0..3: warps x candidates per chunk of the batched BPSW kernel
+ *   MP_TUNE_BPSW_VARIANT   0..3: threads per CTA of the batched base-2 launch
  *   MP_TUNE_FERMAT_ILP2    1: two primes per thread in the Fermat kernel
  * Returns MP_EINVAL for an unknown knob or a value out of range.  No reference counterpart
  * (the reference picks its wheel and chunk by a cost model, A350826/a350826.c:1976-2015). */

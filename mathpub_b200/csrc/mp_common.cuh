@@ -168,7 +168,7 @@ struct Autotune {
     int sieve_tile_log2 = 0;         // 0 = not tuned
     int sieve_threads = 0;
     int fermat_variant = 0;
-    int bpsw_variant = 0;            // warps per CTA x candidates per chunk of the batched BPSW kernel
+    int bpsw_variant = 0;            // threads per CTA of the batched base-2 launch (bpsw_batched_launch)
     int scatter_staged = 1;          // 1: the staged (sorted) bucket scatter, 0: the binned one
     int bucket_div = 1;              // primes above tile bits / bucket_div (1, 2 or 4) go to the bucket scatter
     int no_pipeline = 0;             // 1: batched sieve calls as a host loop of wave launches

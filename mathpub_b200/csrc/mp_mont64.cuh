@@ -11,14 +11,20 @@
 //  * A residue is two 32-bit limbs; each product is one PTX block of 32-bit multiply-add carry
 //    chains, with the subtracting reduction of the 128-bit product t (R = 2^64): m = t n^-1 mod
 //    2^64, then (t - m n) / R = t_hi - hi(m n), exact since the low halves agree, plus n when it
-//    borrows.  In and out in [0, n), for any odd n, and its input may be up to n R, which lets
-//    the doubling below fold into the product for n < 2^63.
-//  * Base-2 exponentiation, left to right, in two size classes (warps run one class at a time):
-//    n < 2^63, one product x (x 2^b) per bit (below 2 n^2 < n R); n >= 2^63, a square, then a
-//    doubling by a funnel shift of the residue by the exponent bit b and one conditional
-//    subtraction (no select between two residues).  (A word-by-word adding reduction with lazy
-//    residues in [0, 2n) for n < 2^62, a square then a doubling per bit, measured 2.5% slower on
-//    the whole batched BPSW than the folded product.)
+//    borrows.  In and out in [0, n), for any odd n.
+//  * Base-2 exponentiation computes 2^-d (the strong test's conditions hold for 2^-d exactly when
+//    they hold for 2^d).  In Montgomery form 2^-c is the plain power of two 2^(64 - c), so the
+//    ladder starts from the top bits of d with a shift, and R mod n is not needed.  Then five
+//    bits at a time: five squarings and one product by 2^-c, c = 0 .. 31, which is a shift left by
+//    32 - c and one word of reduction.  Three size classes, each with its squaring:
+//    n < 2^62 keeps x below 2^63 without a comparison; n < 2^63 with a subtraction of n when bit 63
+//    is set; n >= 2^63 keeps x below 2^64 with a subtraction of n on a carry out.
+//  * The squarings form the cross product once and keep the sums at even and odd words apart,
+//    because a 64-bit multiply-add (mad.lo.cc directly followed by madc.hi.cc) lands in an aligned
+//    pair of registers.  Measured on B200, clocks of an SM per warp: a 64-bit product 1.02, a low
+//    32-bit product 0.51; so n < 2^62 has a floor of 8.2 a squaring and takes 9.5 (n >= 2^63: 14.3,
+//    much of it carries).  A product with the subtracting reduction takes 13.6, and was run for
+//    every bit here before.
 //  * Lucas sequences (P = 1, Q = (1 - D)/4) run as the ladder (V_k, V_k+1, Q^k) with
 //        V_2k = V_k^2 - 2 Q^k,   V_2k+1 = V_k V_k+1 - P Q^k,
 //    the same four products for either exponent bit (the bit only selects operands), so the
@@ -193,38 +199,187 @@ __device__ __forceinline__ u64 mm_from_small(i32 v, const Mod64 &M)
 
 // ---- base-2 strong probable-prime test ----
 
-// size classes of the base-2 ladder: below 2^63 (the doubling folded into the product), 2^63
-// and above (a square, then the doubling)
-#define SP_FOLD 1
-#define SP_WIDE 2
+// size classes of the base-2 ladder: below 2^62 (no corrections), below 2^63, any n
+#define SP_LAZY 1
+#define SP_MID 2
+#define SP_WIDE 3
 
-__device__ __forceinline__ int spsp2_class(u64 n) { return n < (1ull << 63) ? SP_FOLD : SP_WIDE; }
-
-// n - 1 = d 2^s with d odd: 2^d (mod n) by the left-to-right ladder, then the strong
-// condition 2^d = 1, or 2^(d 2^r) = -1 for some 0 <= r < s.  Odd n > 2 in size class CLS.
-template <int CLS>
-__device__ __forceinline__ bool spsp2(const Mod64 &M)
+// x <- x - n when x has bit 63 set
+__device__ __forceinline__ void sp_below63(u32 &x0, u32 &x1, u32 n0, u32 n1)
 {
-    const u64 n = M.n;
-    const int s = __ffsll((long long)(n - 1)) - 1;
-    const u64 d = (n - 1) >> s;
-    const int L = 63 - __clzll((long long)d);               // d's top bit: the ladder starts at 2
-    u64 x = mm_dbl(M.one, 1u, M);
-    for (int i = L - 1; i >= 0; i--) {
-        const u32 bit = (u32)(d >> i) & 1u;
-        if (CLS == SP_FOLD) {
-            x = ms_mul(x, x << bit, M);                     // x (x 2^bit) / R < 2 n^2 / R < n
-        } else {
-            x = ms_sqr(x, M);
-            x = mm_dbl(x, bit, M);
-        }
+    asm("{\n\t.reg .pred p;\n\t"
+        "setp.lt.s32    p, %1, 0;\n\t"
+        "@p sub.cc.u32  %0, %0, %2;\n\t"
+        "@p subc.u32    %1, %1, %3;\n\t}"
+        : "+r"(x0), "+r"(x1) : "r"(n0), "r"(n1));
+}
+
+// x <- x^2 / R (mod n), np = -n^-1 mod 2^32, by two words of adding reduction.
+//   SP_LAZY: x < 2^63, n < 2^62: x^2 / R + n < 2^63, and < 2n once x < 2n
+//   SP_MID:  x < 2^63, n < 2^63: x^2 / R + n < 2^62 + n, less n when that has bit 63 set
+//   SP_WIDE: any x < 2^64: x^2 / R + n < 2^64 + n, less n when it reaches 2^64
+template <int CLS>
+__device__ __forceinline__ void sp_sqr(u32 &x0, u32 &x1, u32 n0, u32 n1, u32 np)
+{
+    if (CLS != SP_WIDE) {
+        asm("{\n\t.reg .u32 a0, a1, a2, a3, b1, b2, e1, m;\n\t"
+            "shl.b32        e1, %1, 1;\n\t"
+            "mul.lo.u32     a0, %0, %0;\n\t"
+            "mul.hi.u32     a1, %0, %0;\n\t"
+            "mul.lo.u32     b1, %0, e1;\n\t"
+            "mul.hi.u32     b2, %0, e1;\n\t"
+            "mul.lo.u32     m, a0, %4;\n\t"
+            "mad.lo.cc.u32  a0, m, %2, a0;\n\t"
+            "madc.hi.cc.u32 a1, m, %2, a1;\n\t"
+            "madc.lo.cc.u32 a2, %1, %1, 0;\n\t"
+            "madc.hi.u32    a3, %1, %1, 0;\n\t"
+            "add.cc.u32     b1, b1, a1;\n\t"
+            "addc.u32       b2, b2, 0;\n\t"
+            "mad.lo.cc.u32  b1, m, %3, b1;\n\t"
+            "madc.hi.cc.u32 b2, m, %3, b2;\n\t"
+            "addc.u32       a3, a3, 0;\n\t"
+            "mul.lo.u32     m, b1, %4;\n\t"
+            "mad.lo.cc.u32  b1, m, %2, b1;\n\t"
+            "madc.hi.cc.u32 b2, m, %2, b2;\n\t"
+            "addc.u32       a3, a3, 0;\n\t"
+            "mad.lo.cc.u32  a2, m, %3, a2;\n\t"
+            "madc.hi.u32    a3, m, %3, a3;\n\t"
+            "add.cc.u32     %0, a2, b2;\n\t"
+            "addc.u32       %1, a3, 0;\n\t}"
+            : "+r"(x0), "+r"(x1) : "r"(n0), "r"(n1), "r"(np));
+        if (CLS == SP_MID) sp_below63(x0, x1, n0, n1);
+    } else {
+        asm("{\n\t.reg .u32 a0, a1, a2, a3, b1, b2, k, m;\n\t.reg .pred p;\n\t"
+            "mul.lo.u32     a0, %0, %0;\n\t"
+            "mul.hi.u32     a1, %0, %0;\n\t"
+            "mul.lo.u32     b1, %0, %1;\n\t"
+            "mul.hi.u32     b2, %0, %1;\n\t"
+            "mul.lo.u32     m, a0, %4;\n\t"
+            "mad.lo.cc.u32  a0, m, %2, a0;\n\t"
+            "madc.hi.cc.u32 a1, m, %2, a1;\n\t"
+            "madc.lo.cc.u32 a2, %1, %1, 0;\n\t"
+            "madc.hi.u32    a3, %1, %1, 0;\n\t"
+            "mad.lo.cc.u32  b1, %0, %1, b1;\n\t"
+            "madc.hi.cc.u32 b2, %0, %1, b2;\n\t"
+            "addc.u32       a3, a3, 0;\n\t"                 // x^2 + m n0 < 2^128
+            "add.cc.u32     b1, b1, a1;\n\t"
+            "addc.cc.u32    b2, b2, 0;\n\t"
+            "addc.cc.u32    a3, a3, 0;\n\t"
+            "addc.u32       k, 0, 0;\n\t"
+            "mad.lo.cc.u32  b1, m, %3, b1;\n\t"
+            "madc.hi.cc.u32 b2, m, %3, b2;\n\t"
+            "addc.cc.u32    a3, a3, 0;\n\t"
+            "addc.u32       k, k, 0;\n\t"
+            "mul.lo.u32     m, b1, %4;\n\t"
+            "mad.lo.cc.u32  b1, m, %2, b1;\n\t"
+            "madc.hi.cc.u32 b2, m, %2, b2;\n\t"
+            "addc.cc.u32    a3, a3, 0;\n\t"
+            "addc.u32       k, k, 0;\n\t"
+            "mad.lo.cc.u32  a2, m, %3, a2;\n\t"
+            "madc.hi.cc.u32 a3, m, %3, a3;\n\t"
+            "addc.u32       k, k, 0;\n\t"
+            "add.cc.u32     %0, a2, b2;\n\t"
+            "addc.cc.u32    %1, a3, 0;\n\t"
+            "addc.u32       k, k, 0;\n\t"
+            "setp.ne.u32    p, k, 0;\n\t"
+            "@p sub.cc.u32  %0, %0, %2;\n\t"
+            "@p subc.u32    %1, %1, %3;\n\t}"
+            : "+r"(x0), "+r"(x1) : "r"(n0), "r"(n1), "r"(np));
     }
-    const u64 mone = n - M.one;                             // the residue of -1
-    bool pass = x == M.one || x == mone;
+}
+
+// x <- (x 2^sh + m n) / 2^32 (mod n), sh in [0, 32]: x itself for 32, else below x / 2 + n; brought
+// into the class's range
+template <int CLS>
+__device__ __forceinline__ void sp_shift(u32 &x0, u32 &x1, u32 sh, u32 n0, u32 n1, u32 np)
+{
+    u32 k;
+    asm("{\n\t.reg .u32 t0, t1, t2, b1, b2, m;\n\t"
+        "shl.b32         t0, %0, %6;\n\t"
+        "shf.l.clamp.b32 t1, %0, %1, %6;\n\t"
+        "shf.l.clamp.b32 t2, %1, 0, %6;\n\t"
+        "mul.lo.u32      m, t0, %5;\n\t"
+        "mul.lo.u32      b1, m, %4;\n\t"
+        "mul.hi.u32      b2, m, %4;\n\t"
+        "mad.lo.cc.u32   t0, m, %3, t0;\n\t"
+        "madc.hi.cc.u32  t1, m, %3, t1;\n\t"
+        "addc.u32        t2, t2, 0;\n\t"                    // below 2^31 + 1
+        "add.cc.u32      %0, t1, b1;\n\t"
+        "addc.cc.u32     %1, t2, b2;\n\t"
+        "addc.u32        %2, 0, 0;\n\t}"
+        : "+r"(x0), "+r"(x1), "=r"(k) : "r"(n0), "r"(n1), "r"(np), "r"(sh));
+    if (CLS == SP_MID) sp_below63(x0, x1, n0, n1);
+    if (CLS == SP_WIDE)
+        asm("{\n\t.reg .pred p;\n\t"
+            "setp.ne.u32    p, %4, 0;\n\t"
+            "@p sub.cc.u32  %0, %0, %2;\n\t"
+            "@p subc.u32    %1, %1, %3;\n\t}"
+            : "+r"(x0), "+r"(x1) : "r"(n0), "r"(n1), "r"(k));
+}
+
+// x / R mod n in [0, n]
+__device__ __forceinline__ u64 sp_leave(u32 x0, u32 x1, u32 n0, u32 n1, u32 np)
+{
+    u32 m = x0 * np;
+    u64 c = (u64)m * n0 + x0;
+    c = (u64)m * n1 + x1 + (c >> 32);
+    const u32 t = (u32)c, u = (u32)(c >> 32);
+    m = t * np;
+    c = (u64)m * n0 + t;
+    return (u64)m * n1 + u + (c >> 32);
+}
+
+// -n^-1 mod 2^32
+__device__ __forceinline__ u32 sp_ninv(u32 n0)
+{
+    u32 v = n0;                                             // n0^-1: 3 bits, doubled four times
+    v *= 2 - n0 * v;
+    v *= 2 - n0 * v;
+    v *= 2 - n0 * v;
+    v *= 2 - n0 * v;
+    return 0u - v;
+}
+
+// x = 2^-d (mod n) in Montgomery form
+template <int CLS>
+__device__ __forceinline__ void sp_ladder(u32 &x0, u32 &x1, u64 d, u64 n, u32 np)
+{
+    const u32 n0 = (u32)n, n1 = (u32)(n >> 32);
+    // w digits of five bits below a top of at most seven: w from the length of n, so that the lanes of
+    // a warp, whose d differ in length, walk the same digits.  The top c: 2^-c R is 2^(64 - c) to
+    // c = 63, one or two more shifts above
+    const int bits = 64 - __clzll((long long)n);
+    int w = bits > 8 ? (bits - 4) / 5 : 0;
+    while (d >> (5 * w) == 0) w--;
+    u32 c = (u32)(d >> (5 * w));
+    u64 x = 1ull << (64 - min(c, 63u));
+    if (CLS != SP_WIDE && d == 1) x -= n;                   // 2^63, brought below 2^63
+    x0 = (u32)x;
+    x1 = (u32)(x >> 32);
+    for (c -= min(c, 63u); c; c -= min(c, 32u)) sp_shift<CLS>(x0, x1, 32u - min(c, 32u), n0, n1, np);
+    while (--w >= 0) {
+#pragma unroll
+        for (int i = 0; i < 5; i++) sp_sqr<CLS>(x0, x1, n0, n1, np);
+        sp_shift<CLS>(x0, x1, 32u - ((u32)(d >> (5 * w)) & 31u), n0, n1, np);
+    }
+}
+
+// n - 1 = d 2^s with d odd: the strong condition 2^-d = 1, or 2^(-d 2^r) = -1 for some
+// 0 <= r < s (mod n).  Odd n > 2 in size class CLS.
+template <int CLS>
+__device__ __forceinline__ bool spsp2(u64 n)
+{
+    const u32 n0 = (u32)n, n1 = (u32)(n >> 32), np = sp_ninv(n0);
+    const int s = __ffsll((long long)(n - 1)) - 1;
+    u32 x0, x1;
+    sp_ladder<CLS>(x0, x1, (n - 1) >> s, n, np);
+    u64 z = sp_leave(x0, x1, n0, n1, np);
+    bool pass = z == 1 || z == n - 1;
     for (int r = 1; r < s && !pass; r++) {
-        if (x == M.one) break;                              // 1 before -1: not a strong probable prime
-        x = ms_sqr(x, M);
-        pass = x == mone;
+        if (z == 1) break;                                  // 1 before -1: not a strong probable prime
+        sp_sqr<CLS>(x0, x1, n0, n1, np);
+        z = sp_leave(x0, x1, n0, n1, np);
+        pass = z == n - 1;
     }
     return pass;
 }
@@ -232,9 +387,7 @@ __device__ __forceinline__ bool spsp2(const Mod64 &M)
 // the test for any odd n > 2, in its size class
 __device__ __forceinline__ bool spsp2_u64(u64 n)
 {
-    const Mod64 M = mm_setup(n);
-    const int c = spsp2_class(n);
-    return c == SP_FOLD ? spsp2<SP_FOLD>(M) : spsp2<SP_WIDE>(M);
+    return n >> 62 == 0 ? spsp2<SP_LAZY>(n) : n >> 63 == 0 ? spsp2<SP_MID>(n) : spsp2<SP_WIDE>(n);
 }
 
 // ---- strong Lucas test ----
@@ -380,10 +533,7 @@ __device__ __forceinline__ bool lucas_u64(u64 n)
 __device__ __forceinline__ bool bpsw_odd(u64 n)
 {
     if (n == ~0ull) return false;
-    const Mod64 M = mm_setup(n);
-    const int c = spsp2_class(n);
-    const bool p2 = c == SP_FOLD ? spsp2<SP_FOLD>(M) : spsp2<SP_WIDE>(M);
-    if (!p2) return false;
+    if (!spsp2_u64(n)) return false;
     const i32 D = selfridge_d(n);
-    return D && lucas_strong(M, D);
+    return D && lucas_strong(mm_setup(n), D);
 }

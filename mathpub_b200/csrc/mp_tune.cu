@@ -1,7 +1,7 @@
 // mp_tune.cu -- the measured autotuner: times the sieve tile geometry (bits per tile x
 // threads per CTA), the bucket scatter's form, the bucket threshold, the batched form
 // (persistent pipeline or wave loop), the Fermat kernel variants (limbs fixed by p, one or two
-// primes per thread) and the batched BPSW kernel's warps per CTA x candidates per queue chunk
+// primes per thread) and the threads per CTA of the batched base-2 test
 // on the device with CUDA events, and keeps the fastest per handle.  The reference
 // chooses its wheel and chunk by a fitted cost model (auto_wheel / auto_chunk,
 // A350826/a350826.c:1976-2015); here the candidates are timed instead.
@@ -122,8 +122,7 @@ extern "C" int mp_autotune(mp_handle *h, uint64_t lo, char *report, size_t cap)
     snprintf(line, sizeof line, "fermat choice: %d prime(s)/thread\n", (fv & 2) ? 2 : 1);
     rep += line;
     // batched BPSW: 2^23 seeded odd candidates (three in four in [2^62, 2^64), the rest in
-    // [2^40, 2^62)), one list, each warps x chunk pair the kernel is built for.  Enough chunks
-    // for several per warp: with fewer CTAs than SMs the launch's tail would decide
+    // [2^40, 2^62)), one list, each CTA size of the base-2 launch
     {
         const u64 cnt = 1ull << 23;
         std::vector<u64> cand(cnt);
