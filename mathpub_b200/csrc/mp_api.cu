@@ -85,7 +85,7 @@ int mp_init(int device, mp_handle **out)
     h->graphs = new GraphCache();
     DevBuf *bufs[] = {&h->tilesum, &h->blockacc, &h->rec, &h->reccnt, &h->queue, &h->errflag, &h->scratch_bitmap,
                       &h->bpsw_n, &h->bpsw_bits, &h->bpsw_list, &h->ferm_p, &h->ferm_q, &h->ferm_part, &h->stats_out, &h->small_out,
-                      &h->boot.q, &h->boot.magic, &h->table.q, &h->table.magic, &h->tstate, &h->gap_acc};
+                      &h->boot.q, &h->boot.magic, &h->table.q, &h->table.magic, &h->tstate, &h->gap_acc, &h->planes, &h->emit_off};
     for (DevBuf *b : bufs) b->gen = &h->buf_gen;
     for (auto &e : h->scat) e.buf.gen = &h->buf_gen;
     *out = h;
@@ -101,11 +101,12 @@ int mp_free(mp_handle *h)
     mp_chain_free(h);
     DevBuf *bufs[] = {&h->tilesum, &h->blockacc, &h->rec, &h->reccnt, &h->queue, &h->errflag, &h->scratch_bitmap,
                       &h->bpsw_n, &h->bpsw_bits, &h->bpsw_list, &h->ferm_p, &h->ferm_q, &h->ferm_part, &h->stats_out, &h->small_out,
-                      &h->boot.q, &h->boot.magic, &h->table.q, &h->table.magic, &h->tstate, &h->gap_acc};
+                      &h->boot.q, &h->boot.magic, &h->table.q, &h->table.magic, &h->tstate, &h->gap_acc, &h->planes, &h->emit_off};
     for (DevBuf *b : bufs) b->release();
     for (auto &e : h->scat) e.buf.release();
     for (int p = 0; p < MP_NPAT; p++)
         if (!h->shared_tables && h->pat_ready && h->pat.d_words[p]) cudaFree(h->pat.d_words[p]);
+    if (!h->shared_tables && h->pat_ready && h->pat.d_words7) cudaFree(h->pat.d_words7);
     if (h->h_err) cudaFreeHost(h->h_err);
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);

@@ -150,6 +150,8 @@ struct PatternSet {
     u32 period[MP_NPAT];
     u64 words[MP_NPAT];              // u32 words stored per pattern
     u32 *d_words[MP_NPAT];
+    u32 period7;                     // 7 11 13 17 19: the first pattern without 3 and 5
+    u32 *d_words7;
 };
 
 // odd sieving primes 3 <= q <= limit with Barrett constants, resident on the device; a host
@@ -207,7 +209,7 @@ struct mp_handle {
 
     // scratch
     DevBuf tilesum, blockacc, rec, reccnt, queue, errflag, scratch_bitmap, bpsw_n, bpsw_bits, bpsw_list,
-        ferm_p, ferm_q, ferm_part, stats_out, small_out, tstate, gap_acc;
+        ferm_p, ferm_q, ferm_part, stats_out, small_out, tstate, gap_acc, planes, emit_off;
     // CTA bounds of the bucket scatter, one buffer per (first prime, end prime, CTAs): a
     // captured graph reads the buffer it was captured with, so a buffer's contents are never
     // rewritten; the least recently used one is freed (which invalidates the graphs) when a

@@ -24,7 +24,7 @@
 // A tile summary (count, twins, tuples, checksum, first/last prime, widest internal gap)
 // goes to HBM; a one-CTA fold kernel joins the summaries in order into block and range
 // results, attributing every gap to the prime that starts it.
-#include "mp_common.cuh"
+#include "mp_sieve.cuh"
 #include <algorithm>
 #include <math.h>
 #include <stdarg.h>
@@ -44,21 +44,6 @@ static const u32 kPatPrimes[MP_NPAT][7] = {
     {3, 5, 7, 11, 13, 17, 19}, {23, 29, 31, 37, 0}, {41, 43, 47, 53, 0}, {59, 61, 67, 71, 0}, {73, 79, 83, 89, 0}};
 __constant__ u32 c_pat_primes[MP_NPAT][7] = {
     {3, 5, 7, 11, 13, 17, 19}, {23, 29, 31, 37, 0}, {41, 43, 47, 53, 0}, {59, 61, 67, 71, 0}, {73, 79, 83, 89, 0}};
-
-struct TileSum {
-    u64 first, last;   // first / last prime bit in the tile (bits < nbx); MP_NONE if none
-    u64 lastin;        // last prime bit below limit; MP_NONE if none
-    u64 mgs;           // bit of the prime starting the widest internal gap; MP_NONE if none
-    u64 cks;           // sum of mix64(p) over the 6-tuple starts p (bits < limit)
-    u32 mg;            // widest internal gap in bits (pairs whose first prime is in range)
-    u32 count;         // primes with bit < limit
-    u32 twins, tuples;
-};
-
-struct SieveGeom {
-    u64 base, limit, nbx;   // base even; bits [0, limit) in range; bits [0, nbx) sieved
-    u32 tlog, ntiles;
-};
 
 struct TileArgs {
     SieveGeom g;
@@ -93,85 +78,8 @@ struct Wave {
 #define W30_FAR (1u << 28)
 
 // ---------------------------------------------------------------------------------------
-// ordered combine of tile / thread summaries
-// ---------------------------------------------------------------------------------------
-
-struct Part {
-    u64 first, last, lastin, mgs, cks;
-    u32 mg, count, twins, tuples;
-};
-
-__device__ __forceinline__ void part_init(Part &p)
-{
-    p.first = p.last = p.lastin = p.mgs = MP_NONE;
-    p.cks = 0;
-    p.mg = p.count = p.twins = p.tuples = 0;
-}
-
-// L followed by R (R's bits all above L's); gaps compare strictly so the earliest start wins
-__device__ __forceinline__ Part part_join(const Part &L, const Part &R, u64 limit)
-{
-    Part o;
-    o.count = L.count + R.count;
-    o.twins = L.twins + R.twins;
-    o.tuples = L.tuples + R.tuples;
-    o.cks = L.cks + R.cks;
-    o.mg = L.mg;
-    o.mgs = L.mgs;
-    if (L.first == MP_NONE) {
-        o.first = R.first; o.last = R.last; o.lastin = R.lastin; o.mg = R.mg; o.mgs = R.mgs;
-        return o;
-    }
-    o.first = L.first;
-    if (R.first == MP_NONE) { o.last = L.last; o.lastin = L.lastin; return o; }
-    o.last = R.last;
-    o.lastin = R.lastin != MP_NONE ? R.lastin : L.lastin;
-    if (L.last < limit) {
-        const u32 g = (u32)(R.first - L.last);
-        if (g > o.mg) { o.mg = g; o.mgs = L.last; }
-    }
-    if (R.mg > o.mg) { o.mg = R.mg; o.mgs = R.mgs; }
-    return o;
-}
-
-__device__ __forceinline__ Part part_shfl_down(const Part &p, int d)
-{
-    Part o;
-    o.first = __shfl_down_sync(0xffffffffu, p.first, d);
-    o.last = __shfl_down_sync(0xffffffffu, p.last, d);
-    o.lastin = __shfl_down_sync(0xffffffffu, p.lastin, d);
-    o.mgs = __shfl_down_sync(0xffffffffu, p.mgs, d);
-    o.cks = __shfl_down_sync(0xffffffffu, p.cks, d);
-    o.mg = __shfl_down_sync(0xffffffffu, p.mg, d);
-    o.count = __shfl_down_sync(0xffffffffu, p.count, d);
-    o.twins = __shfl_down_sync(0xffffffffu, p.twins, d);
-    o.tuples = __shfl_down_sync(0xffffffffu, p.tuples, d);
-    return o;
-}
-
-// in-order reduction over the lanes of a warp; lane 0 holds the result
-__device__ __forceinline__ Part part_warp_reduce(Part p, u64 limit)
-{
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        Part r = part_shfl_down(p, d);
-        if ((lane & (2 * d - 1)) == 0) p = part_join(p, r, limit);
-    }
-    return p;
-}
-
-// ---------------------------------------------------------------------------------------
 // tile kernel
 // ---------------------------------------------------------------------------------------
-
-__device__ __forceinline__ u32 bits_mask(u64 start, u64 bound)
-{
-    // bits start .. start+31 below bound
-    if (start >= bound) return 0;
-    const u64 n = bound - start;
-    return n >= 32 ? 0xffffffffu : ((1u << n) - 1);
-}
 
 // a 16-byte bucket-record load: streaming through L1 in a kernel of its own, through L2 only
 // inside the pipeline kernel
@@ -1436,7 +1344,7 @@ u64 PrimeTable::count_le(u64 x) const
 int mp_patterns_ensure(mp_handle *h)
 {
     if (h->pat_ready) return MP_OK;
-    const u64 slack_bits = (1ull << MAX_TLOG) + HALO_BITS + 8 * 32 + 256;
+    const u64 slack_bits = (1ull << (MAX_TLOG + 1)) + HALO_BITS + 8 * 32 + 256;   // past a tile's bits
     for (int p = 0; p < MP_NPAT; p++) {
         u64 per = 1;
         for (int k = 0; k < 7 && kPatPrimes[p][k]; k++) per *= kPatPrimes[p][k];
@@ -1448,6 +1356,11 @@ int mp_patterns_ensure(mp_handle *h)
         pattern_kernel<<<1024, 256, 0, h->stream>>>(h->pat.d_words[p], words, Q[0], Q[1], Q[2], Q[3], Q[4], Q[5], Q[6]);
         MP_CUDA(h, cudaGetLastError());
     }
+    h->pat.period7 = 7 * 11 * 13 * 17 * 19;
+    const u64 words7 = (h->pat.period7 + slack_bits) / 32 + 16;
+    MP_CUDA(h, cudaMalloc(&h->pat.d_words7, words7 * 4));
+    pattern_kernel<<<1024, 256, 0, h->stream>>>(h->pat.d_words7, words7, 7, 11, 13, 17, 19, 0, 0);
+    MP_CUDA(h, cudaGetLastError());
     MP_CUDA(h, cudaStreamSynchronize(h->stream));
     h->pat_ready = true;
     return MP_OK;
@@ -1958,6 +1871,30 @@ static int pick_geometry(mp_handle *h, const mp_sieve_opts *o, u32 &tlog, int &n
     return MP_OK;
 }
 
+// whether a batched call runs in residue planes (mp_planes.cu): unless the call or the handle pins a
+// geometry or form of the odd-only tiles
+static bool planes_form(const mp_handle *h, const mp_sieve_opts *o)
+{
+    return !(o && (o->tile_log2 || o->threads)) && !h->tune.sieve_tile_log2 && !h->tune.sieve_threads &&
+           h->tune.scatter_staged == 1 && h->tune.bucket_div == 1;
+}
+
+// the range and its stretches: 2^20 bits, fewer for ranges that would leave SMs without one, and no
+// more than a block
+static int planes_geom(mp_handle *h, u64 lo, u64 hi, u32 block_log2, SieveGeom &g)
+{
+    g.base = lo & ~1ull;
+    g.limit = (hi - g.base) >> 1;
+    g.nbx = (hi + MP_TAIL - g.base) >> 1;
+    g.tlog = 20;
+    while (g.tlog > 14 && (g.nbx >> g.tlog) < 2 * (u64)h->sm_count) g.tlog--;
+    if (block_log2 && g.tlog > block_log2 - 1) g.tlog = block_log2 - 1;
+    const u64 n = (g.nbx + (1ull << g.tlog) - 1) >> g.tlog;
+    if (n >= (1ull << 31)) return mp_set_error(h, MP_ERANGE, "range too long (%llu tiles)", (unsigned long long)n);
+    g.ntiles = (u32)n;
+    return MP_OK;
+}
+
 int mp_sieve_run(mp_handle *h, u64 lo, u64 hi, const mp_sieve_opts *o, mp_range_stats *d_out,
                  mp_block_stats *d_blocks, u64 *d_hash, u64 *d_bitmap, cudaStream_t st)
 {
@@ -1978,7 +1915,10 @@ int mp_sieve_run(mp_handle *h, u64 lo, u64 hi, const mp_sieve_opts *o, mp_range_
     const u64 top = hi + MP_TAIL;
     MP_TRY(mp_tables_ensure(h, mp_isqrt64(top - 1)));
     SievePlan P;
-    MP_TRY(plan_sieve(h, *h->tab, lo, hi, tlog, nth, P));
+    const bool planes = mode == MP_MODE_BATCHED && planes_form(h, o);
+    if (planes) MP_TRY(planes_geom(h, lo, hi, block_log2, P.g));
+    else MP_TRY(plan_sieve(h, *h->tab, lo, hi, tlog, nth, P));
+    tlog = P.g.tlog;
     MP_CUDA(h, h->tilesum.ensure((size_t)P.g.ntiles * sizeof(TileSum)));
     // bitmap: the caller's, or scratch when only hashes are wanted
     const u64 nwords64 = (P.g.limit + 63) >> 6;
@@ -1987,11 +1927,15 @@ int mp_sieve_run(mp_handle *h, u64 lo, u64 hi, const mp_sieve_opts *o, mp_range_
         MP_CUDA(h, h->scratch_bitmap.ensure((size_t)nwords64 * 8 + 64));
         bm = h->scratch_bitmap.as<u32>();
     }
-    TileArgs a;
-    fill_tile_args(h, *h->tab, P, a);
-    a.sums = h->tilesum.as<TileSum>();
-    a.bitmap32 = bm;
-    MP_TRY(run_tiles(h, *h->tab, P, a, (int)mode, 0, st));
+    if (planes) {
+        MP_TRY(mp_planes_run(h, *h->tab, P.g, h->tilesum.as<TileSum>(), bm, nullptr, 0, nullptr, st));
+    } else {
+        TileArgs a;
+        fill_tile_args(h, *h->tab, P, a);
+        a.sums = h->tilesum.as<TileSum>();
+        a.bitmap32 = bm;
+        MP_TRY(run_tiles(h, *h->tab, P, a, (int)mode, 0, st));
+    }
     // fold
     u32 tpb;
     u64 nblocks;
@@ -2010,7 +1954,7 @@ int mp_sieve_run(mp_handle *h, u64 lo, u64 hi, const mp_sieve_opts *o, mp_range_
     MP_CUDA(h, h->blockacc.ensure((size_t)nbe * sizeof(Part)));
     FoldArgs f;
     f.base = P.g.base; f.limit = P.g.limit; f.lo = lo; f.hi = hi;
-    f.sums = a.sums; f.ntiles = P.g.ntiles; f.tpb = tpb;
+    f.sums = h->tilesum.as<TileSum>(); f.ntiles = P.g.ntiles; f.tpb = tpb;
     f.nblocks = (u32)std::min<u64>(nblocks, nbe); f.nblocks_ext = (u32)nbe;
     f.acc = h->blockacc.as<Part>();
     f.out = d_out; f.blocks = d_blocks; f.err = h->errflag.as<u32>();
@@ -2042,6 +1986,27 @@ int mp_sieve_emit_primes(mp_handle *h, u64 lo, u64 hi, u64 *d_primes, u64 cap, u
     MP_TRY(pick_geometry(h, nullptr, tlog, nth));
     const u64 top = hi + MP_TAIL;
     MP_TRY(mp_tables_ensure(h, mp_isqrt64(top - 1)));
+    if (planes_form(h, nullptr)) {
+        // counted and written in one pass: the primes past cap are counted only
+        SieveGeom g;
+        MP_TRY(planes_geom(h, lo, hi, 0, g));
+        MP_CUDA(h, h->tilesum.ensure((size_t)g.ntiles * sizeof(TileSum)));
+        MP_CUDA(h, h->small_out.ensure(256));
+        u64 *total = h->small_out.as<u64>() + 24;
+        const u64 has2 = lo <= 2 && 2 < hi;
+        if (has2 && d_primes && cap) {
+            const u64 two = 2;
+            MP_CUDA(h, cudaMemcpyAsync(d_primes, &two, 8, cudaMemcpyHostToDevice, st));
+        }
+        const bool put = d_primes && cap > has2;
+        MP_TRY(mp_planes_run(h, *h->tab, g, h->tilesum.as<TileSum>(), nullptr, put ? d_primes + has2 : nullptr,
+                             put ? cap - has2 : 0, total, st));
+        u64 n = 0;
+        MP_CUDA(h, cudaMemcpyAsync(&n, total, 8, cudaMemcpyDeviceToHost, st));
+        MP_TRY(check_errflag(h, st));                                      // synchronises
+        *count = n + has2;
+        return MP_OK;
+    }
     SievePlan P;
     MP_TRY(plan_sieve(h, *h->tab, lo, hi, tlog, nth, P));
     MP_CUDA(h, h->tilesum.ensure((size_t)P.g.ntiles * sizeof(TileSum)));
