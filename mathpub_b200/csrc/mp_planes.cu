@@ -231,7 +231,7 @@ struct PlaneScatterArgs {
     const u32 *q;
     const u64 *magic;
     u32 k0, k1;                       // the bucket primes
-    u32 run;                          // primes a warp takes from the queue at once
+    u32 kc, run;                      // primes a warp takes from the queue at once: 32 below kc, then run
     u32 *rec, *cnt;                   // [8 nb][cap], [8 nb] zeroed before the launch
     u32 cap;
     u32 *queue;                       // zeroed before the launch
@@ -241,7 +241,17 @@ struct PlaneScatterArgs {
 #define PS_THREADS 512
 #define PS_STAGE 8192                 // staged records per CTA (two buffers of them)
 #define PS_CTAS_PER_SM 3
+#ifndef PS_TRIES
+#define PS_TRIES 1
+#endif
+#ifndef QBN
+#define QBN 4
+#endif
+#ifndef QWMAX
+#define QWMAX 8192
+#endif
 #define PS_OFF_BITS 21                // staged record: tile << 21 | offset
+#define PS_NONE 0xffffffffu           // an empty place of the stage
 
 // sort the staged records by tile and write them to their buckets (all threads)
 __device__ __forceinline__ void plane_flush(const PlaneScatterArgs &a, u32 nt, u32 *stage, u32 *sorted, u32 *hist,
@@ -272,6 +282,7 @@ __device__ __forceinline__ void plane_flush(const PlaneScatterArgs &a, u32 nt, u
             if (lane >= (u32)d) iv += u;
         }
         if (lane < PS_THREADS / 32) s_wsum[lane] = iv - v;
+        if (lane == PS_THREADS / 32 - 1) s_wsum[PS_THREADS / 32] = iv;    // all records
     }
     __syncthreads();
     // reserve each tile's run in its bucket; hist becomes the placement cursor and gb the
@@ -290,11 +301,12 @@ __device__ __forceinline__ void plane_flush(const PlaneScatterArgs &a, u32 nt, u
     __syncthreads();
     for (u32 i = tid; i < n; i += PS_THREADS) {
         const u32 r = stage[i];
-        sorted[atomicAdd(&hist[r >> PS_OFF_BITS], 1u)] = r;
+        if (r != PS_NONE) sorted[atomicAdd(&hist[r >> PS_OFF_BITS], 1u)] = r;
     }
+    const u32 nrec = s_wsum[PS_THREADS / 32];
     __syncthreads();
     // the runs of one tile are consecutive in sorted order and in the bucket
-    for (u32 i = tid; i < n; i += PS_THREADS) {
+    for (u32 i = tid; i < nrec; i += PS_THREADS) {
         const u32 r = sorted[i], tl = r >> PS_OFF_BITS, slot = gb[tl] + i;
         if (slot < a.cap) __stcs(a.rec + (u64)tl * a.cap + slot, r & ((1u << PS_OFF_BITS) - 1u));
     }
@@ -315,7 +327,7 @@ __global__ void __launch_bounds__(PS_THREADS, PS_CTAS_PER_SM) plane_scatter_kern
     const u32 nt = 8 * a.nb;
     u32 *stage = ssm, *sorted = ssm + PS_STAGE, *hist = ssm + 2 * PS_STAGE, *gb = hist + nt;
     __shared__ u32 s_fill;
-    __shared__ u32 s_wsum[PS_THREADS / 32];
+    __shared__ u32 s_wsum[PS_THREADS / 32 + 1];
     __shared__ __align__(8) u64 s_u[30], s_v[30];        // u and v of the eight planes, a byte each, by q mod 30
     const u32 tid = threadIdx.x, lane = tid & 31, lt = (1u << lane) - 1;
     for (u32 i = tid; i < nt; i += PS_THREADS) hist[i] = 0;
@@ -330,7 +342,7 @@ __global__ void __launch_bounds__(PS_THREADS, PS_CTAS_PER_SM) plane_scatter_kern
         s_u[tid] = U;
         s_v[tid] = V;
     }
-    const u32 ni = a.ni, pt = a.pt, nb = a.nb;
+    const u32 ni = a.ni, pt = a.pt, nb = a.nb, dense_q = ni / 2;
     u32 jj[8], q = 0;
     bool have = false;
     u32 wk = 0, wend = 0;                                // the warp's run of primes
@@ -338,16 +350,18 @@ __global__ void __launch_bounds__(PS_THREADS, PS_CTAS_PER_SM) plane_scatter_kern
     __syncthreads();
     for (;;) {
         // hand out primes; a prime without a hit in the wave is dropped on the spot
-        for (int tries = 0; tries < 4; tries++) {
+        for (int tries = 0; tries < PS_TRIES; tries++) {
             const u32 need = __ballot_sync(0xffffffffu, !have);
             if (!need) break;
             if (wk >= wend) {
                 if (dry) break;
                 u32 c = 0;
-                if (lane == 0) c = atomicAdd(a.queue, a.run);
+                if (lane == 0) c = atomicAdd(a.queue, 1u);
                 c = __shfl_sync(0xffffffffu, c, 0);
-                wk = c < a.k1 - a.k0 ? a.k0 + c : a.k1;
-                wend = min(wk + a.run, a.k1);
+                const u32 fine = (a.kc - a.k0) >> 5;     // kc - k0 is a multiple of 32
+                const u64 k = c < fine ? a.k0 + 32ull * c : a.kc + (u64)a.run * (c - fine);
+                wk = (u32)min(k, (u64)a.k1);
+                wend = min(wk + (c < fine ? 32u : a.run), a.k1);
                 dry = wk >= a.k1;
                 if (dry) break;
             }
@@ -377,37 +391,54 @@ __global__ void __launch_bounds__(PS_THREADS, PS_CTAS_PER_SM) plane_scatter_kern
         const u32 fill = s_fill;
         __syncthreads();
         if (fill > PS_STAGE - 8 * PS_THREADS) plane_flush(a, nt, stage, sorted, hist, gb, &s_fill, s_wsum);
-        u32 rec[8], nmine = 0, jmin = 0xffffffffu;
+        // one hit per plane: rec = tile << 21 | bit in the tile, as blk (2^21 - pt) + j + (plane nb << 21)
+        u32 rec[8], jmin = 0xffffffffu;
 #pragma unroll
         for (int i = 0; i < 8; i++) {
             const u32 j = jj[i];
             const bool v = have && j < ni;
-            const u32 blk = __umulhi(j >> 10, a.blk_magic);
-            rec[i] = v ? ((i * nb + blk) << PS_OFF_BITS) | (j - blk * pt) : 0xffffffffu;
-            nmine += v;
-            const u32 jn = v ? j + q : 0xffffffffu;
-            jj[i] = jn < j ? 0xffffffffu : jn;           // no wrap: q may be close to 2^32
+            rec[i] = v ? __umulhi(j >> 10, a.blk_magic) * ((1u << PS_OFF_BITS) - pt) + (j + i * (nb << PS_OFF_BITS))
+                       : PS_NONE;
+            const u32 jn = v ? j + q : PS_NONE;
+            jj[i] = jn < j ? PS_NONE : jn;               // no wrap: q may be close to 2^32
             jmin = min(jmin, jj[i]);
         }
-        have = have && jmin < ni;
-        // warp-aggregated append to the stage
-        u32 incl = nmine;
+        if (__all_sync(0xffffffffu, have && q <= dense_q)) {
+            // nearly every place is taken: the lane's eight go down as they are, empty ones marked
+            u32 base = 0;
+            if (lane == 0) base = atomicAdd(&s_fill, 256u);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            uint4 *const at = (uint4 *)(stage + base + 8 * lane);
+            at[0] = make_uint4(rec[0], rec[1], rec[2], rec[3]);
+            at[1] = make_uint4(rec[4], rec[5], rec[6], rec[7]);
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const u32 u = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane >= (u32)d) incl += u;
-        }
-        u32 base = 0;
-        if (lane == 31 && incl) base = atomicAdd(&s_fill, incl);
-        base = __shfl_sync(0xffffffffu, base, 31);
-        u32 pos = base + incl - nmine;
+            for (int i = 0; i < 8; i++)
+                if (rec[i] != PS_NONE) atomicAdd(&hist[rec[i] >> PS_OFF_BITS], 1u);
+        } else {
+            u32 nmine = 0;
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            if (rec[i] != 0xffffffffu) {
-                stage[pos++] = rec[i];
-                atomicAdd(&hist[rec[i] >> PS_OFF_BITS], 1u);
+            for (int i = 0; i < 8; i++) nmine += rec[i] != PS_NONE;
+            u32 incl = nmine;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const u32 u = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= (u32)d) incl += u;
+            }
+            const u32 tot = __shfl_sync(0xffffffffu, incl, 31), res = (tot + 3) & ~3u;   // 16-byte steps
+            u32 base = 0;
+            if (lane == 0 && tot) base = atomicAdd(&s_fill, res);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            u32 pos = base + incl - nmine;
+            if (lane < res - tot) stage[base + tot + lane] = PS_NONE;
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                if (rec[i] != PS_NONE) {
+                    stage[pos++] = rec[i];
+                    atomicAdd(&hist[rec[i] >> PS_OFF_BITS], 1u);
+                }
             }
         }
+        have = have && jmin < ni;
     }
     plane_flush(a, nt, stage, sorted, hist, gb, &s_fill, s_wsum);
 }
@@ -992,8 +1023,8 @@ static int plan_planes(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, P
         // tiers: a prime has pt / q multiples in a tile
         P.iend = (u32)tb.count_le(sq);
         P.iw0 = (u32)std::min<u64>(tb.count_le(89), P.iend);
-        P.iw1 = std::max(P.iw0, (u32)std::min<u64>(tb.count_le(std::min<u32>(8192, P.pt / 64)), P.iend));
-        P.it1 = std::max(P.iw1, (u32)std::min<u64>(tb.count_le(P.pt), P.iend));
+        P.iw1 = std::max(P.iw0, (u32)std::min<u64>(tb.count_le(std::min<u32>(QWMAX, P.pt / 64)), P.iend));
+        P.it1 = std::max(P.iw1, (u32)std::min<u64>(tb.count_le((u64)P.pt * QBN / 4), P.iend));
         P.cap = 0;
         if (P.iend > P.it1) {
             // expected records of a tile: each bucket prime hits a block of pt bits pt / q times
@@ -1076,8 +1107,11 @@ int mp_planes_run(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, TileSu
             s.q = a.q; s.magic = a.magic;
             s.k0 = P.it1; s.k1 = P.iend;
             const u32 nblk = (u32)h->sm_count * PS_CTAS_PER_SM;
-            // runs of 32 .. 512 primes: several per warp, and few enough that the queue is no bottleneck
-            s.run = std::max(32u, std::min(512u, (s.k1 - s.k0) / (nblk * (PS_THREADS / 32) * 8) & ~31u));
+            // runs of 32 primes where they take several rounds, then up to 512, so that the queue is no
+            // bottleneck and no warp is left with a long run (measured: runs of 512 throughout, 6.4 ms
+            // instead of 2.2 at 9e17, where a few warps held the smallest primes)
+            s.kc = s.k0 + (std::min(s.k1, std::max(s.k0, (u32)tb.count_le(s.ni / 4))) - s.k0 & ~31u);
+            s.run = std::max(32u, std::min(512u, (s.k1 - s.kc) / (nblk * (PS_THREADS / 32) * 8) & ~31u));
             s.rec = h->rec.as<u32>(); s.cnt = h->reccnt.as<u32>(); s.cap = P.cap;
             s.queue = s.cnt + ntile;
             s.err = h->errflag.as<u32>();
