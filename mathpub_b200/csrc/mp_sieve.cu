@@ -1111,6 +1111,25 @@ __device__ __forceinline__ void racc_join(RangeAcc &r, const RangeAcc &B)
     if (B.mgs != MP_NONE && (r.mgs == MP_NONE || B.mg > r.mg)) { r.mg = B.mg; r.mgs = B.mgs; }
 }
 
+// in-order join over the lanes of a warp; lane 0 holds the result
+__device__ __forceinline__ void racc_warp_join(RangeAcc &r)
+{
+    const u32 lane = threadIdx.x & 31;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        RangeAcc o;
+        o.n = __shfl_down_sync(0xffffffffu, r.n, d);
+        o.tw = __shfl_down_sync(0xffffffffu, r.tw, d);
+        o.tu = __shfl_down_sync(0xffffffffu, r.tu, d);
+        o.cks = __shfl_down_sync(0xffffffffu, r.cks, d);
+        o.first = __shfl_down_sync(0xffffffffu, r.first, d);
+        o.lastin = __shfl_down_sync(0xffffffffu, r.lastin, d);
+        o.mgs = __shfl_down_sync(0xffffffffu, r.mgs, d);
+        o.mg = __shfl_down_sync(0xffffffffu, r.mg, d);
+        if ((lane & (2 * d - 1)) == 0) racc_join(r, o);
+    }
+}
+
 // 64-bit totals: block parts carry u32 counts (a block is at most 2^31 bits); the range
 // total is summed in 64 bits
 __global__ void __launch_bounds__(512) fold_kernel(FoldArgs a)
@@ -1161,20 +1180,25 @@ __global__ void __launch_bounds__(512) fold_kernel(FoldArgs a)
         }
     }
     // 4. range: in-order join of the in-range blocks, whose parts already hold their
-    //    trailing gaps (each thread a contiguous run of blocks, then thread 0 in order)
-    __shared__ RangeAcc s_r[512];
+    //    trailing gaps: each thread a contiguous run of blocks, then the threads by shuffles (one
+    //    thread joining the 512 took 20 us)
+    __shared__ RangeAcc s_r[16];
+    const u32 lane = tid & 31;
+    RangeAcc R;
     {
         const u32 per = (a.nblocks + nth - 1) / nth;
-        RangeAcc R;
         racc_init(R);
         for (u32 b = tid * per; b < (tid + 1) * per && b < a.nblocks; b++) racc_add(R, a.acc[b]);
-        s_r[tid] = R;
+        racc_warp_join(R);
+        if (lane == 0) s_r[tid >> 5] = R;
     }
     __syncthreads();
-    if (tid == 0) {
-        RangeAcc R;
+    if (tid < 32) {
         racc_init(R);
-        for (u32 i = 0; i < nth; i++) racc_join(R, s_r[i]);
+        if (lane < nth / 32) R = s_r[lane];
+        racc_warp_join(R);
+    }
+    if (tid == 0) {
         mp_range_stats o;
         o.pi = R.n;
         o.twins = R.tw;
@@ -1195,68 +1219,240 @@ __global__ void __launch_bounds__(512) fold_kernel(FoldArgs a)
 }
 
 // ---------------------------------------------------------------------------------------
-// FNV-1a-64 per hash segment of the bitmap.  The hash is a serial chain over the segment's
-// bytes, so each thread hashes one segment; one warp per CTA spreads the segments over every
-// SM.  Each thread keeps HASH_AHEAD 16-byte loads (256 bytes) in flight ahead of its chain,
-// which otherwise waits on every load.
+// FNV-1a-64 per hash segment of the bitmap: h <- (h ^ byte) P, P = 2^40 + 435, a serial chain.  Two
+// forms, chosen by the number of segments (hash_launch).
+//
+// One thread per segment, one warp per CTA to spread the segments over every SM.  A step on 32-bit halves: x = lo ^ byte,
+// lo <- low(435 x), hi <- 435 hi + high(435 x) + 256 x, the two last products as multiply-adds, so that
+// the chain is one XOR and one 32 x 32 -> 64 product long: 15.5 cycles a byte on B200 (the 64-bit
+// product 21.2; the low half alone, which nothing can shorten, 11.5).  16384 segments of 64 KB:
+// 0.66 -> 0.57 ms.
 // ---------------------------------------------------------------------------------------
 
-#define HASH_AHEAD 16
+#define HASH_AHEAD 16                 // 16-byte words of a segment per stage
+#define HASH_PITCH (HASH_AHEAD + 1)   // of a stage's rows, so that the lanes' reads meet no bank twice
 
-__device__ __forceinline__ void fnv_word(u64 &h, u32 w)
-{
+struct Fnv {
+    u32 lo, hi;
+    __device__ __forceinline__ void byte(u32 e)
+    {
+        const u32 x = lo ^ e;
+        asm("{\n\t.reg .u64 p;\n\t.reg .u32 h, c;\n\t"
+            "mul.wide.u32 p, %2, 435;\n\t"
+            "mov.b64 {%0, h}, p;\n\t"
+            "mad.lo.u32 c, %2, 256, h;\n\t"
+            "mad.lo.u32 %1, %1, 435, c;\n\t}"
+            : "=&r"(lo), "+r"(hi) : "r"(x));
+    }
+    __device__ __forceinline__ void word(u32 w)
+    {
 #pragma unroll
-    for (int j = 0; j < 4; j++) { h ^= (w >> (8 * j)) & 0xffu; h *= MP_FNV_PRIME; }
-}
-
-__device__ __forceinline__ void fnv_16(u64 &h, const uint4 v)
-{
-    fnv_word(h, v.x); fnv_word(h, v.y); fnv_word(h, v.z); fnv_word(h, v.w);
-}
+        for (int j = 0; j < 4; j++) byte(__byte_perm(w, 0, 0x4440 + j));
+    }
+    __device__ __forceinline__ void quad(const uint4 v) { word(v.x); word(v.y); word(v.z); word(v.w); }
+    __device__ __forceinline__ u64 value() const { return (u64)hi << 32 | lo; }
+};
 
 __global__ void __launch_bounds__(32) hash_kernel(const u32 *__restrict__ bm, u64 nbits, u64 seg_bits, u64 nseg,
                                                   u64 *out)
 {
+    __shared__ uint4 stage[2][32 * HASH_PITCH];
     const u64 s = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nseg) return;
+    const u32 lane = threadIdx.x;
     const u64 b0 = s * seg_bits;
-    const u64 len = b0 + seg_bits <= nbits ? seg_bits : nbits - b0;
+    const u64 len = s >= nseg ? 0 : b0 + seg_bits <= nbits ? seg_bits : nbits - b0;   // lanes past the end: empty
     const u64 nbytes = (len + 7) >> 3;
     const u8 *p = (const u8 *)bm + (b0 >> 3);       // seg_bits is a multiple of 8
-    u64 h = MP_FNV_OFFSET;
+    Fnv h{(u32)MP_FNV_OFFSET, (u32)(MP_FNV_OFFSET >> 32)};
     u64 k = 0;
     // bytes up to a 16-byte boundary (all but the last byte of the segment are whole)
-    for (; k + 1 < nbytes && (((uintptr_t)(p + k)) & 15); k++) { h ^= p[k]; h *= MP_FNV_PRIME; }
-    // whole blocks of HASH_AHEAD 16-byte words: the loads of block b + 1 are issued while
-    // block b is hashed
+    for (; k + 1 < nbytes && (((uintptr_t)(p + k)) & 15); k++) h.byte(p[k]);
+    // whole blocks of HASH_AHEAD 16-byte words.  Each lane copies its block b + 1 to shared memory
+    // (asynchronously) while block b is hashed from there: with plain loads the chains waited on them,
+    // 32 sectors a load (0.72 ms instead of 0.57)
     const u64 nblk = nbytes > k + 1 ? (nbytes - k - 1) / (16 * HASH_AHEAD) : 0;
-    if (nblk) {
-        const uint4 *v = (const uint4 *)(p + k);
-        uint4 buf[HASH_AHEAD];
+    const bool rows = (seg_bits & 127) == 0 && ((uintptr_t)bm & 15) == 0;        // then k = 0 everywhere
+    if (rows) {
+        const u32 most = __reduce_max_sync(0xffffffffu, (u32)nblk);
+        const u32 to = (u32)__cvta_generic_to_shared(&stage[0][lane * HASH_PITCH]);
+        const auto fetch = [&](u32 b) {
+            if (b < nblk)
 #pragma unroll
-        for (int i = 0; i < HASH_AHEAD; i++) buf[i] = __ldcs(v + i);
-        for (u64 b = 0; b < nblk; b++) {
-            const uint4 *nx = v + (b + 1) * HASH_AHEAD;
-            const bool more = b + 1 < nblk;
-#pragma unroll
-            for (int i = 0; i < HASH_AHEAD; i++) {
-                const uint4 x = buf[i];
-                if (more) buf[i] = __ldcs(nx + i);
-                fnv_16(h, x);
-            }
+                for (u32 i = 0; i < HASH_AHEAD; i++)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::
+                                 "r"(to + (b & 1) * (32 * HASH_PITCH * 16) + 16 * i), "l"(p + 16 * (HASH_AHEAD * (u64)b + i))
+                                 : "memory");
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        fetch(0);
+        for (u32 b = 0; b < most; b++) {
+            fetch(b + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            if (b < nblk)
+#pragma unroll 8
+                for (int i = 0; i < HASH_AHEAD; i++) h.quad(stage[b & 1][lane * HASH_PITCH + i]);
         }
         k += nblk * 16 * HASH_AHEAD;
     }
     // the rest in 16-byte words while one byte more remains, then bytes; the last byte keeps
     // only the bits of the segment
-    for (; k + 16 < nbytes; k += 16) fnv_16(h, __ldcs((const uint4 *)(p + k)));
+    if (((uintptr_t)(p + k) & 15) == 0)
+        for (; k + 16 < nbytes; k += 16) h.quad(__ldcs((const uint4 *)(p + k)));
     for (; k < nbytes; k++) {
         u8 c = p[k];
         const u64 rem = len - 8 * k;
         if (rem < 8) c &= (u8)((1u << rem) - 1);
-        h ^= c; h *= MP_FNV_PRIME;
+        h.byte(c);
     }
-    out[s] = h;
+    if (s < nseg) out[s] = h.value();
+}
+
+// The parallel form, one warp per segment, 1024 bytes a row, 32 consecutive bytes a lane.  Only the low
+// byte l of the state meets the data: h ^ b = h + ((l ^ b) - l), so given l at the start of a stretch
+// of v bytes, its chain run from h = l alone gives d = chain - l P^v, and h <- h P^v + d: the
+// stretches join linearly.  And l follows x = l ^ b, l <- 179 x (mod 256): bit k of 179 x is x_k plus
+// a carry of lower bits, so bit k of l is a running XOR of known bits once the lower bits of every
+// position are known.  Eight prefix XORs over the row, bit by bit from the lowest, give l at every
+// lane's start.  About 200 cycles of an SM per row against 15.5 a byte and thread for the serial form,
+// which therefore wins from about 11,000 segments on.
+__device__ __forceinline__ u32 prefix_xor(u32 g)
+{
+    g ^= g << 1;
+    g ^= g << 2;
+    g ^= g << 4;
+    g ^= g << 8;
+    return g ^ (g << 16);
+}
+
+__device__ __forceinline__ u64 fnv_pow(u64 e)              // P^e
+{
+    u64 r = 1, b = MP_FNV_PRIME;
+    for (; e; e >>= 1, b *= b)
+        if (e & 1) r *= b;
+    return r;
+}
+
+// full adder on bit slices: sum and carry
+__device__ __forceinline__ u32 fa_sum(u32 a, u32 b, u32 c) { return a ^ b ^ c; }
+__device__ __forceinline__ u32 fa_carry(u32 a, u32 b, u32 c) { return (a & b) | (c & (a | b)); }
+
+// s[k]: bit k of the lane's 32 bytes, bit p of it for byte p.  state: the row's first low byte, replaced
+// by the one after the row.  Returns the low byte at the lane's first byte
+__device__ __forceinline__ u32 row_states(const u32 (&s)[8], u32 &state)
+{
+    const u32 lane = threadIdx.x & 31;
+    u32 L = 0, next = 0, x[8];
+    const auto level = [&](int k, u32 r) {                 // r: the carry of the lower bits into bit k
+        const u32 g = prefix_xor(s[k] ^ r);
+        const u32 pm = prefix_xor(__ballot_sync(0xffffffffu, g >> 31));
+        const u32 st = ((lane ? pm >> (lane - 1) : 0u) ^ (state >> k)) & 1u;
+        next |= ((pm >> 31) ^ (state >> k) & 1u) << k;
+        L |= st << k;
+        x[k] = (g << 1) ^ (0u - st) ^ s[k];
+    };
+    // 179 = 1 + 2 + 16 + 32 + 128: bit k of 179 x adds x_k, x_k-1, x_k-4, x_k-5, x_k-7 and carries
+    level(0, 0);
+    level(1, x[0]);
+    const u32 c2 = x[1] & x[0];
+    level(2, x[1] ^ c2);
+    const u32 c3 = fa_carry(x[2], x[1], c2);
+    level(3, x[2] ^ c3);
+    const u32 c4 = fa_carry(x[3], x[2], c3);
+    level(4, x[3] ^ x[0] ^ c4);
+    const u32 t4 = fa_sum(x[4], x[3], x[0]), c5 = fa_carry(x[4], x[3], x[0]), d5 = t4 & c4;
+    level(5, x[4] ^ x[1] ^ x[0] ^ c5 ^ d5);
+    const u32 t5 = fa_sum(x[5], x[4], x[1]), c6 = fa_carry(x[5], x[4], x[1]);
+    const u32 u5 = fa_sum(x[0], c5, d5), d6 = fa_carry(x[0], c5, d5), e6 = t5 & u5;
+    level(6, x[5] ^ x[2] ^ x[1] ^ c6 ^ d6 ^ e6);
+    const u32 t6 = fa_sum(x[6], x[5], x[2]), c7 = fa_carry(x[6], x[5], x[2]);
+    const u32 u6 = fa_sum(x[1], c6, d6), d7 = fa_carry(x[1], c6, d6), e7 = fa_carry(t6, u6, e6);
+    level(7, x[6] ^ x[3] ^ x[2] ^ x[0] ^ c7 ^ d7 ^ e7);
+    state = next;
+    return L;
+}
+
+__global__ void __launch_bounds__(128) hash_rows_kernel(const u32 *__restrict__ bm, u64 nbits, u64 seg_bits, u64 nseg,
+                                                        u64 *out)
+{
+    const u64 sg = (u64)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (sg >= nseg) return;                                // the warp's lanes leave together
+    const u32 lane = threadIdx.x & 31;
+    const u64 b0 = sg * seg_bits;
+    const u64 len = b0 + seg_bits <= nbits ? seg_bits : nbits - b0;
+    const u64 nbytes = (len + 7) >> 3, rows = nbytes >> 10;
+    const u32 rem = (u32)(nbytes & 1023);
+    const u64 *p = (const u64 *)((const u8 *)bm + (b0 >> 3)) + 4 * lane;   // segments are whole 64-bit words
+    u32 state = (u32)MP_FNV_OFFSET & 0xffu;
+    const u64 P32 = fnv_pow(32), P1024 = fnv_pow(1024);
+    u64 acc = 0, tail = 0, buf[4];
+    const auto fetch = [&](u64 row) {
+        const u64 at = row * 1024 + lane * 32;
+#pragma unroll
+        for (int k = 0; k < 4; k++) buf[k] = at + 8 * k < nbytes ? __ldcs(p + row * 128 + k) : 0ull;
+    };
+    fetch(0);
+    for (u64 row = 0; row < rows + (rem != 0); row++) {
+        u32 w[8], s[8];
+#pragma unroll
+        for (int k = 0; k < 4; k++) { w[2 * k] = (u32)buf[k]; w[2 * k + 1] = (u32)(buf[k] >> 32); }
+        fetch(row + 1);
+        const u32 v = row < rows ? 32u : (u32)max(0, min(32, (int)rem - 32 * (int)lane));
+        if (row == rows && v && (len & 7) && 32 * lane + v == rem) {      // the last byte keeps its bits only
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+                if (k == (int)((v - 1) >> 2)) w[k] &= ~0u >> (8 * (3 - ((v - 1) & 3)) + 8 - (u32)(len & 7));
+        }
+        // 32 bytes -> 8 slices: 8 x 8 bit transposes, then the bytes of each slice together
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            u32 x = w[2 * i], y = w[2 * i + 1], t;
+            t = (x ^ (x >> 7)) & 0x00AA00AAu;
+            x ^= t ^ (t << 7);
+            t = (x ^ (x >> 14)) & 0x0000CCCCu;
+            x ^= t ^ (t << 14);
+            t = (y ^ (y >> 7)) & 0x00AA00AAu;
+            y ^= t ^ (t << 7);
+            t = (y ^ (y >> 14)) & 0x0000CCCCu;
+            y ^= t ^ (t << 14);
+            t = (x ^ (y << 4)) & 0xF0F0F0F0u;
+            s[2 * i] = x ^ t;
+            s[2 * i + 1] = y ^ (t >> 4);
+        }
+        u32 sl[8];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const u32 a = __byte_perm(s[h], s[2 + h], 0x5140), b = __byte_perm(s[h], s[2 + h], 0x7362);
+            const u32 c = __byte_perm(s[4 + h], s[6 + h], 0x5140), d = __byte_perm(s[4 + h], s[6 + h], 0x7362);
+            sl[4 * h] = __byte_perm(a, c, 0x5410);
+            sl[4 * h + 1] = __byte_perm(a, c, 0x7632);
+            sl[4 * h + 2] = __byte_perm(b, d, 0x5410);
+            sl[4 * h + 3] = __byte_perm(b, d, 0x7632);
+        }
+        const u32 L = row_states(sl, state);
+        Fnv h{L, 0};
+        if (row < rows) {
+#pragma unroll
+            for (int k = 0; k < 8; k++) h.word(w[k]);
+            acc = acc * P1024 + (h.value() - L * P32);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 32; k++)
+                if (k < (int)v) h.byte(__byte_perm(w[k >> 2], 0, 0x4440 + (k & 3)));
+            tail = (h.value() - L * fnv_pow(v)) * fnv_pow(v ? rem - 32 * lane - v : 0);
+        }
+    }
+    acc = acc * fnv_pow(32 * (31 - lane)) * fnv_pow(rem) + tail;
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
+    if (lane == 0) out[sg] = MP_FNV_OFFSET * fnv_pow(nbytes) + acc;
+}
+
+static void hash_launch(const u32 *bm, u64 nbits, u64 seg_bits, u64 nseg, u64 *out, cudaStream_t st)
+{
+    // the parallel form for segments of a row and more, up to the count where it takes as long as the
+    // serial one (whose time does not depend on the count while each has a thread of its own)
+    if (seg_bits >= 8192 && nseg <= 11000) hash_rows_kernel<<<(unsigned)((nseg + 3) / 4), 128, 0, st>>>(bm, nbits, seg_bits, nseg, out);
+    else hash_kernel<<<(unsigned)((nseg + 31) / 32), 32, 0, st>>>(bm, nbits, seg_bits, nseg, out);
 }
 
 // exclusive prefix of tile counts -> emit offsets; total to *total (one CTA)
@@ -1968,7 +2164,7 @@ int mp_sieve_run(mp_handle *h, u64 lo, u64 hi, const mp_sieve_opts *o, mp_range_
         const u64 sb = 1ull << (hash_log2 - 1);
         const u64 ns = (P.g.limit + sb - 1) / sb;
         ProfScope ps(h, PROF_HASH, st);
-        hash_kernel<<<(unsigned)((ns + 31) / 32), 32, 0, st>>>(bm, P.g.limit, sb, ns, d_hash);
+        hash_launch(bm, P.g.limit, sb, ns, d_hash, st);
         MP_CUDA(h, cudaGetLastError());
     }
     return MP_OK;
