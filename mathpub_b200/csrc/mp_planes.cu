@@ -41,6 +41,7 @@ __host__ __device__ __forceinline__ PlaneUV pl_uv(u32 r, u32 c)
 
 #define PL_PTMAX 1769472u             // bits of a tile at most (216 KB of shared memory)
 #define PL_NPAT MP_NPAT
+#define PL_IMOD_MIN 4096u            // primes from which on a launch for their remainders pays
 
 struct PlaneTileArgs {
     u64 i0;                           // index of the wave's first plane bit
@@ -54,18 +55,36 @@ struct PlaneTileArgs {
     u32 cap;
     u32 *planes;                      // [8][nb pt / 32] words, set bits are primes
     u32 *tstate;                      // per CTA: next multiple of each thread-tier prime
+    const u32 *imod;                  // i0 mod q for the primes from iw0 on (nullable)
 };
 
-// index (relative to `is`) of the first multiple of q at or after `is` in the CTA's plane, the
-// prime q itself excepted; uv: the plane's table by q mod 30
-__device__ __forceinline__ u32 plane_first(u64 is, u32 q, u64 magic, const u16 *uv)
+// index (relative to is) of the first multiple of q at or after `is` in the CTA's plane, the prime
+// itself excepted, from m = is mod q; uv: the plane's table by q mod 30
+__device__ __forceinline__ u32 plane_first(u64 is, u32 q, u32 m, const u16 *uv)
 {
-    const u32 m = mp_mod_barrett(is, q, magic);
     const u32 a = q / 30u, t = uv[q - 30u * a], u = t & 0xffu;
     const u32 s = a * u + (t >> 8);                      // < q
-    u32 j = s - m + (s < m ? q : 0u);
+    u32 j = s - m;
+    j = min(j, j + q);                                   // s < m: below zero, so the sum is the smaller
     if (is <= a && u == 1 && is + j == a) j += q;
     return j;
+}
+
+// (i0 + off) mod q from r = i0 mod q, which a launch of its own took once for the wave, and M = floor(2^32
+// / q): a 32-bit remainder instead of a 64-bit one.  r + off < 2^32: q < 2^21, off < 2^31
+__device__ __forceinline__ u32 plane_mod(u32 r, u32 off, u32 q, u32 M)
+{
+    const u32 x = r + off;
+    u32 m = x - __umulhi(x, M) * q;                      // < 3 q
+    m = min(m, m - q);
+    return min(m, m - q);
+}
+
+__global__ void __launch_bounds__(256) plane_imod_kernel(const u32 *__restrict__ q, const u64 *__restrict__ magic, u32 n,
+                                                         u64 i0, u32 *__restrict__ out)
+{
+    const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = mp_mod_barrett(i0, q[i], magic[i]);
 }
 
 __device__ __forceinline__ void plane_presieve(u32 *sm, u32 nw, const PlaneTileArgs &a, const u32 *s_off)
@@ -103,12 +122,14 @@ __device__ __forceinline__ void plane_presieve(u32 *sm, u32 nw, const PlaneTileA
 
 // CTA b sieves the tiles [b per, (b + 1) per) of the wave in order; tile t is block t mod nb of
 // plane t / nb, so that the thread-tier primes carry their next multiple along a plane
-__global__ void __launch_bounds__(1024) plane_tile_kernel(PlaneTileArgs a)
+template <int NTH>
+__global__ void __launch_bounds__(NTH) plane_tile_kernel(PlaneTileArgs a)
 {
     extern __shared__ __align__(16) u32 sm[];            // pt / 32 words
     __shared__ u32 s_off[PL_NPAT];
     __shared__ u16 s_uv[30];
-    const u32 tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nth >> 5;
+    const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr u32 nth = NTH, nwarps = NTH / 32;
     const u32 pt = a.pt, nw = pt >> 5;
     const u32 per = (a.ntile + gridDim.x - 1) / gridDim.x;
     const u32 tb = blockIdx.x * per, te = min(tb + per, a.ntile);
@@ -139,75 +160,134 @@ __global__ void __launch_bounds__(1024) plane_tile_kernel(PlaneTileArgs a)
                 }
             if (is == 0 && pl == 0) atomicOr(&sm[0], 1u);
         }
-        // warp tier.  Warp w takes the primes w, w + nwarps, ... of the tier, 32 at a time: lane i
-        // sets up prime i of the batch, then the warp marks the batch one prime after the other,
-        // lane l the multiples l, l + 32, ...: 32 q bits apart, so a lane's mask stays and its word
-        // advances by q
-        for (u32 kb = a.iw0 + warp; kb < a.iw1; kb += 32 * nwarps) {
-            const u32 k = kb + nwarps * lane;
-            u32 q = 0, j = 0;
-            if (k < a.iw1) {
-                q = __ldg(a.q + k);
-                j = plane_first(is, q, __ldg(a.magic + k), s_uv);
-            }
-            const u32 n = min(32u, (a.iw1 - kb + nwarps - 1) / nwarps);
-            for (u32 i = 0; i < n; i++) {
-                const u32 qi = __shfl_sync(0xffffffffu, q, i), ji = __shfl_sync(0xffffffffu, j, i) + lane * qi;
-                const u32 m = __funnelshift_l(0u, 1u, ji);
-                u32 w = ji >> 5;
-                for (; w + 3 * qi < nw; w += 4 * qi) {
-                    atomicOr(&sm[w], m);
-                    atomicOr(&sm[w + qi], m);
-                    atomicOr(&sm[w + 2 * qi], m);
-                    atomicOr(&sm[w + 3 * qi], m);
+        // The marks, in any order: the warp tier is bound by shared memory, the thread tier and the
+        // records by L2, so a third of the warps starts with each ([1e15, +2^34): 3.44 ms of tile kernel
+        // against 3.79 with every warp in the same order; by warp & 1 3.53)
+        for (u32 step = 0; step < 3; step++) {
+            const u32 part = (step + warp) % 3u;
+            if (part == 0) {
+                // warp tier.  Warp w takes the primes w, w + nwarps, ... of the tier, 32 at a time: lane i
+                // sets up prime i of the batch, then the warp marks the batch one prime after the other,
+                // lane l the multiples l, l + 32, ...: 32 q bits apart, so a lane's mask stays and its word
+                // advances by q
+                for (u32 kb = a.iw0 + warp; kb < a.iw1; kb += 32 * nwarps) {
+                    const u32 k = kb + nwarps * lane;
+                    u32 q = 0, j = 0;
+                    if (k < a.iw1) {
+                        q = __ldg(a.q + k);
+                        const u64 M = __ldg(a.magic + k);
+                        const u32 m = a.imod ? plane_mod(__ldg(a.imod + (k - a.iw0)), blk * pt, q, (u32)(M >> 32))
+                                             : mp_mod_barrett(is, q, M);
+                        j = plane_first(is, q, m, s_uv);
+                    }
+                    const u32 n = min(32u, (a.iw1 - kb + nwarps - 1) / nwarps);
+                    for (u32 i = 0; i < n; i++) {
+                        const u32 qi = __shfl_sync(0xffffffffu, q, i), ji = __shfl_sync(0xffffffffu, j, i) + lane * qi;
+                        const u32 m = __funnelshift_l(0u, 1u, ji);
+                        u32 w = ji >> 5;
+                        if (33 * qi <= nw) {
+                            // at least 32 steps a lane: the lanes start at different steps, lane l at the one
+                            // whose word is in bank l (q is odd), go to the end and on from the first word, so
+                            // that a step meets each bank once, twice while some lanes have wrapped
+                            u32 inv = qi;
+                            inv *= 2 - qi * inv;                  // 1 / q mod 64
+                            const u32 first = w, start = w + qi * (((lane - w) * inv) & 31u);
+                            w = start;
+                            do {
+                                atomicOr(&sm[w], m);
+                                w += qi;
+                                if (w >= nw) w = first;
+                            } while (w != start);
+                            continue;
+                        }
+                        for (; w + 3 * qi < nw; w += 4 * qi) {
+                            atomicOr(&sm[w], m);
+                            atomicOr(&sm[w + qi], m);
+                            atomicOr(&sm[w + 2 * qi], m);
+                            atomicOr(&sm[w + 3 * qi], m);
+                        }
+                        for (; w < nw; w += qi) atomicOr(&sm[w], m);
+                    }
                 }
-                for (; w < nw; w += qi) atomicOr(&sm[w], m);
-            }
-        }
-        // thread tier, one thread per prime, its next multiple carried to the plane's next block;
-        // eight primes per thread are loaded ahead
-        for (u32 k = a.iw1 + tid; k < a.it1; k += 8 * nth) {
-            u32 qv[8], jv[8];
+            } else if (part == 1) {
+                // thread tier, one thread per prime, its next multiple carried to the plane's next block.  Half
+                // of a visit was address arithmetic and bounds, so the thread count is a constant (the eight
+                // primes a thread loads ahead are immediate offsets) and whole batches run without checks
+                {
+                    const u32 n = a.it1 - a.iw1;
+                    const u32 *pq = a.q + a.iw1 + tid;
+                    u32 *ps = tst + tid;
+                    u32 i = tid;
+                    if (!fresh) {
+                        for (; i + 7 * NTH < n; i += 8 * NTH, pq += 8 * NTH, ps += 8 * NTH) {
+                            u32 qv[8], jv[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const u32 kk = k + u * nth;
-                qv[u] = kk < a.it1 ? __ldg(a.q + kk) : 0u;
-                jv[u] = (kk < a.it1 && !fresh) ? tst[kk - a.iw1] : 0u;
-            }
+                            for (int u = 0; u < 8; u++) {
+                                qv[u] = __ldg(pq + u * NTH);
+                                jv[u] = ps[u * NTH];
+                            }
 #pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const u32 q = qv[u], kk = k + u * nth;
-                if (!q) continue;
-                u32 j = fresh ? plane_first(is, q, __ldg(a.magic + kk), s_uv) : jv[u];
-                for (; j < pt; j += q) atomicOr(&sm[j >> 5], __funnelshift_l(0u, 1u, j));
-                if (keep) tst[kk - a.iw1] = j - pt;
-            }
-        }
-        // bucket records of this tile: read once, with streaming hints
-        if (a.rec) {
-            const u32 n = min(__ldg(a.cnt + t), a.cap);
-            const u32 *R = a.rec + (u64)t * a.cap;       // cap is a multiple of 4
-            const uint4 *R4 = (const uint4 *)R;
-            const u32 n4 = n >> 2;
-            u32 i = tid;
-            for (; i + 3 * nth < n4; i += 4 * nth) {     // 16 records in flight per thread
-                const uint4 r0 = __ldcs(R4 + i), r1 = __ldcs(R4 + i + nth);
-                const uint4 r2 = __ldcs(R4 + i + 2 * nth), r3 = __ldcs(R4 + i + 3 * nth);
-                const u32 js[16] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w,
-                                    r2.x, r2.y, r2.z, r2.w, r3.x, r3.y, r3.z, r3.w};
+                            for (int u = 0; u < 8; u++) {
+                                u32 j = jv[u];
+                                for (; j < pt; j += qv[u]) atomicOr(&sm[j >> 5], __funnelshift_l(0u, 1u, j));
+                                if (keep) ps[u * NTH] = j - pt;
+                            }
+                        }
+                    } else if (a.imod) {
+                        const u32 *pr = a.imod + (a.iw1 - a.iw0) + i, *pm = (const u32 *)(a.magic + a.iw1 + i) + 1;
+                        for (; i + 3 * NTH < n; i += 4 * NTH, pq += 4 * NTH, ps += 4 * NTH, pr += 4 * NTH, pm += 8 * NTH) {
+                            u32 qv[4], jv[4], mv[4];
 #pragma unroll
-                for (int k = 0; k < 16; k++) atomicOr(&sm[js[k] >> 5], __funnelshift_l(0u, 1u, js[k]));
-            }
-            for (; i < n4; i += nth) {
-                const uint4 r0 = __ldcs(R4 + i);
-                atomicOr(&sm[r0.x >> 5], __funnelshift_l(0u, 1u, r0.x));
-                atomicOr(&sm[r0.y >> 5], __funnelshift_l(0u, 1u, r0.y));
-                atomicOr(&sm[r0.z >> 5], __funnelshift_l(0u, 1u, r0.z));
-                atomicOr(&sm[r0.w >> 5], __funnelshift_l(0u, 1u, r0.w));
-            }
-            for (u32 k = (n4 << 2) + tid; k < n; k += nth) {
-                const u32 j = __ldcs(R + k);
-                atomicOr(&sm[j >> 5], __funnelshift_l(0u, 1u, j));
+                            for (int u = 0; u < 4; u++) {
+                                qv[u] = __ldg(pq + u * NTH);
+                                jv[u] = __ldg(pr + u * NTH);
+                                mv[u] = __ldg(pm + 2 * u * NTH);
+                            }
+#pragma unroll
+                            for (int u = 0; u < 4; u++) {
+                                u32 j = plane_first(is, qv[u], plane_mod(jv[u], blk * pt, qv[u], mv[u]), s_uv);
+                                for (; j < pt; j += qv[u]) atomicOr(&sm[j >> 5], __funnelshift_l(0u, 1u, j));
+                                if (keep) ps[u * NTH] = j - pt;
+                            }
+                        }
+                    }
+                    for (; i < n; i += NTH, pq += NTH, ps += NTH) {
+                        const u32 q = __ldg(pq);
+                        u32 j;
+                        if (!fresh) j = *ps;
+                        else j = plane_first(is, q, mp_mod_barrett(is, q, __ldg(a.magic + a.iw1 + i)), s_uv);
+                        for (; j < pt; j += q) atomicOr(&sm[j >> 5], __funnelshift_l(0u, 1u, j));
+                        if (keep) *ps = j - pt;
+                    }
+                }
+            } else if (a.rec) {
+                // bucket records of this tile: read once, with streaming hints
+                {
+                    const u32 n = min(__ldg(a.cnt + t), a.cap);
+                    const u32 *R = a.rec + (u64)t * a.cap;       // cap is a multiple of 4
+                    const uint4 *R4 = (const uint4 *)R;
+                    const u32 n4 = n >> 2;
+                    u32 i = tid;
+                    for (; i + 3 * nth < n4; i += 4 * nth) {     // 16 records in flight per thread
+                        const uint4 r0 = __ldcs(R4 + i), r1 = __ldcs(R4 + i + nth);
+                        const uint4 r2 = __ldcs(R4 + i + 2 * nth), r3 = __ldcs(R4 + i + 3 * nth);
+                        const u32 js[16] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w,
+                                            r2.x, r2.y, r2.z, r2.w, r3.x, r3.y, r3.z, r3.w};
+#pragma unroll
+                        for (int k = 0; k < 16; k++) atomicOr(&sm[js[k] >> 5], __funnelshift_l(0u, 1u, js[k]));
+                    }
+                    for (; i < n4; i += nth) {
+                        const uint4 r0 = __ldcs(R4 + i);
+                        atomicOr(&sm[r0.x >> 5], __funnelshift_l(0u, 1u, r0.x));
+                        atomicOr(&sm[r0.y >> 5], __funnelshift_l(0u, 1u, r0.y));
+                        atomicOr(&sm[r0.z >> 5], __funnelshift_l(0u, 1u, r0.z));
+                        atomicOr(&sm[r0.w >> 5], __funnelshift_l(0u, 1u, r0.w));
+                    }
+                    for (u32 k = (n4 << 2) + tid; k < n; k += nth) {
+                        const u32 j = __ldcs(R + k);
+                        atomicOr(&sm[j >> 5], __funnelshift_l(0u, 1u, j));
+                    }
+                }
             }
         }
         __syncthreads();
@@ -241,15 +321,6 @@ struct PlaneScatterArgs {
 #define PS_THREADS 512
 #define PS_STAGE 8192                 // staged records per CTA (two buffers of them)
 #define PS_CTAS_PER_SM 3
-#ifndef PS_TRIES
-#define PS_TRIES 1
-#endif
-#ifndef QBN
-#define QBN 4
-#endif
-#ifndef QWMAX
-#define QWMAX 8192
-#endif
 #define PS_OFF_BITS 21                // staged record: tile << 21 | offset
 #define PS_NONE 0xffffffffu           // an empty place of the stage
 
@@ -349,22 +420,20 @@ __global__ void __launch_bounds__(PS_THREADS, PS_CTAS_PER_SM) plane_scatter_kern
     bool dry = false;                                    // the queue is empty
     __syncthreads();
     for (;;) {
-        // hand out primes; a prime without a hit in the wave is dropped on the spot
-        for (int tries = 0; tries < PS_TRIES; tries++) {
-            const u32 need = __ballot_sync(0xffffffffu, !have);
-            if (!need) break;
-            if (wk >= wend) {
-                if (dry) break;
-                u32 c = 0;
-                if (lane == 0) c = atomicAdd(a.queue, 1u);
-                c = __shfl_sync(0xffffffffu, c, 0);
-                const u32 fine = (a.kc - a.k0) >> 5;     // kc - k0 is a multiple of 32
-                const u64 k = c < fine ? a.k0 + 32ull * c : a.kc + (u64)a.run * (c - fine);
-                wk = (u32)min(k, (u64)a.k1);
-                wend = min(wk + (c < fine ? 32u : a.run), a.k1);
-                dry = wk >= a.k1;
-                if (dry) break;
-            }
+        // hand out primes to the lanes that have none; a prime without a hit is dropped on the spot, its
+        // lane tries again in the next round
+        const u32 need = __ballot_sync(0xffffffffu, !have);
+        if (need && wk >= wend && !dry) {
+            u32 c = 0;
+            if (lane == 0) c = atomicAdd(a.queue, 1u);
+            c = __shfl_sync(0xffffffffu, c, 0);
+            const u32 fine = (a.kc - a.k0) >> 5;         // kc - k0 is a multiple of 32
+            const u64 k = c < fine ? a.k0 + 32ull * c : a.kc + (u64)a.run * (c - fine);
+            wk = (u32)min(k, (u64)a.k1);
+            wend = min(wk + (c < fine ? 32u : a.run), a.k1);
+            dry = wk >= a.k1;
+        }
+        if (need && wk < wend) {
             const u32 k = wk + __popc(need & lt);
             if (!have && k < wend) {
                 q = __ldg(a.q + k);
@@ -460,7 +529,7 @@ struct PlaneScanArgs {
     u64 emit_cap;
 };
 
-#define SCAN_WARPS 8
+#define SCAN_WARPS 8                  // warps per CTA at most
 
 // the stretch's numbers x, A < x < E (x < base + 2 nbx), as index ranges of the planes relative to i0,
 // and the part of them below the range's end
@@ -608,19 +677,22 @@ __device__ __forceinline__ u32 run_starts(u32 any, u32 next, bool prev, u32 Z)
 // between 30 z + 2 and 30 z + 58, so once a gap of g is known only runs of at least (g - 28) / 30
 // empty blocks are looked at, which are rare.  Until that is at least 1 the row's primes are walked.
 template <bool BITMAP>
-__global__ void __launch_bounds__(32 * SCAN_WARPS) plane_scan_kernel(PlaneScanArgs a)
+__global__ void __launch_bounds__(32 * SCAN_WARPS, 2) plane_scan_kernel(PlaneScanArgs a)
 {
     __shared__ Stretch S;
     __shared__ Part s_part[SCAN_WARPS];
     __shared__ u16 s_odds[BITMAP ? 256 : 1];
     __shared__ u32 s_row[BITMAP ? SCAN_WARPS : 1][BITMAP ? 481 : 1];
-    const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __shared__ u32 s_best;              // the CTA's widest gap
+    const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
     const u32 t = a.t0 + blockIdx.x;
     const u64 base = a.g.base, i0 = a.i0;
-    if (BITMAP) s_odds[tid] = (u16)block_odds(tid);
+    if (tid == 0) s_best = 0;
+    if (BITMAP)
+        for (u32 i = tid; i < 256; i += blockDim.x) s_odds[i] = (u16)block_odds(i);
     stretch_setup(S, a, t);
     const u64 LIM = S.LIM;
-    const u32 nrow = (S.w1 - S.w0 + 31) / 32, wrow = (nrow + SCAN_WARPS - 1) / SCAN_WARPS;
+    const u32 nrow = (S.w1 - S.w0 + 31) / 32, wrow = (nrow + nwarps - 1) / nwarps;
     const u32 c0 = min(S.w0 + warp * wrow * 32, S.w1), c1 = min(c0 + wrow * 32, S.w1);
     const u32 *const P0 = a.planes;
     u32 cnt = 0, tw = 0, tu = 0, bg = 0, fw = ~0u, lw = 0, liw = 0;     // lw, liw: word + 1
@@ -725,7 +797,11 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS) plane_scan_kernel(PlaneScanAr
             }
         };
         const auto reduce_best = [&] {
-            best = max(best, __reduce_max_sync(0xffffffffu, bg));
+            const u32 r = __reduce_max_sync(0xffffffffu, bg);
+            if (r > best) {
+                best = r;
+                if (lane == 0) atomicMax(&s_best, r);
+            }
         };
         if (best < 58) {
             // the longest runs of the row first, which settles the threshold at once at most heights
@@ -781,7 +857,9 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS) plane_scan_kernel(PlaneScanAr
             walked = walk || !rl;
         }
         if (!walk) {
-            const u32 st = run_starts(any, nxt, prev, min(32u, (best - 28) / 30));
+            // a gap found by another warp counts too, but one that ties it may come first here
+            const u32 other = *(volatile u32 *)&s_best, Z = max(best - 28, other > 30 ? other - 30 : 0u) / 30;
+            const u32 st = run_starts(any, nxt, prev, min(32u, Z));
             if (__any_sync(0xffffffffu, st != 0)) {
                 close_runs(st);
                 __syncwarp();
@@ -807,6 +885,13 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS) plane_scan_kernel(PlaneScanAr
             const u64 G = (u64)t << a.g.tlog;
             const i64 m0 = (i64)(G >> 5), m1 = (i64)((min(G + (1ull << a.g.tlog), (a.g.limit + 63) & ~63ull) + 31) >> 5);
             const u32 nk = 15 * min(32u, c1 - wr);
+            const i64 mr = (i64)15 * wr + dq;             // the row's first map word
+            if (nk == 480 && mr > 0 && mr >= m0 && mr + 480 <= m1 && (u64)(mr + 480) * 32 <= a.g.limit) {
+                u32 *const out = a.bitmap32 + mr + lane;
+#pragma unroll
+                for (u32 k = 0; k < 15; k++)
+                    out[32 * k] = __funnelshift_l(row[32 * k + lane], row[32 * k + lane + 1], ds);
+            } else
             for (u32 k = lane; k < nk; k += 32) {
                 const i64 m = (i64)15 * wr + k + dq;
                 if (m < m0 || m >= m1) continue;
@@ -861,7 +946,7 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS) plane_scan_kernel(PlaneScanAr
     __syncthreads();
     if (warp == 0) {
         Part Q;
-        if (lane < SCAN_WARPS) Q = s_part[lane];
+        if (lane < nwarps) Q = s_part[lane];
         else part_init(Q);
         Q = part_warp_reduce(Q, a.g.limit);
         if (lane == 0) {
@@ -1020,11 +1105,13 @@ static int plan_planes(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, P
         if (nb > 4 * group && P.tw > 1) continue;
         P.nb = (u32)((P.ni + P.pt - 1) / P.pt);
         P.threads = P.pt >= (1u << 19) ? 1024 : P.pt >= (1u << 17) ? 512 : 256;
-        // tiers: a prime has pt / q multiples in a tile
+        // tiers: a prime has pt / q multiples in a tile.  The buckets start at 1.5 pt: a visit of a prime
+        // that often misses costs a thread less than its hits cost the scatter ([1e15, +2^34): 1.0 pt 7.60,
+        // 1.25 pt 7.57, 1.5 pt 7.52, 1.75 pt 7.61, 2 pt 7.66 ms a call)
         P.iend = (u32)tb.count_le(sq);
         P.iw0 = (u32)std::min<u64>(tb.count_le(89), P.iend);
-        P.iw1 = std::max(P.iw0, (u32)std::min<u64>(tb.count_le(std::min<u32>(QWMAX, P.pt / 64)), P.iend));
-        P.it1 = std::max(P.iw1, (u32)std::min<u64>(tb.count_le((u64)P.pt * QBN / 4), P.iend));
+        P.iw1 = std::max(P.iw0, (u32)std::min<u64>(tb.count_le(std::min<u32>(8192, P.pt / 64)), P.iend));
+        P.it1 = std::max(P.iw1, (u32)std::min<u64>(tb.count_le((u64)P.pt * 3 / 2), P.iend));
         P.cap = 0;
         if (P.iend > P.it1) {
             // expected records of a tile: each bucket prime hits a block of pt bits pt / q times
@@ -1040,19 +1127,22 @@ static int plan_planes(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, P
 int mp_planes_run(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, TileSum *sums, u32 *bitmap32, u64 *emit,
                   u64 emit_cap, u64 *emit_total, cudaStream_t st)
 {
-    static bool tile_done[16] = {false}, scat_done[16] = {false};
+    static bool tile_done[3][16] = {{false}}, scat_done[16] = {false};
     PlanePlan P;
     MP_TRY(plan_planes(h, tb, g, P));
     int smem_max = 0;
     MP_CUDA(h, cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
-    MP_CUDA(h, raise_smem(plane_tile_kernel, tile_done, h->device, (int)(PL_PTMAX / 8)));
+    const int tk = P.threads == 1024 ? 2 : P.threads == 512 ? 1 : 0;
+    static void (*const tile[3])(PlaneTileArgs) = {plane_tile_kernel<256>, plane_tile_kernel<512>, plane_tile_kernel<1024>};
+    MP_CUDA(h, raise_smem(tile[tk], tile_done[tk], h->device, (int)(PL_PTMAX / 8)));
     const u32 ntile = 8 * P.nb, nw = P.pt / 32;
     const size_t tsm = P.pt / 8;
     int occ = 0;
-    MP_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, plane_tile_kernel, (int)P.threads, tsm));
+    MP_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, tile[tk], (int)P.threads, tsm));
     const u32 grid = (u32)std::min<u64>(ntile, (u64)h->sm_count * (u32)std::max(occ, 1));
     MP_CUDA(h, h->planes.ensure(((size_t)ntile * nw + 64) * 4));
-    MP_CUDA(h, h->tstate.ensure((size_t)grid * (P.it1 - P.iw1) * 4 + 64));
+    const u32 nmod = P.it1 - P.iw0 >= PL_IMOD_MIN ? P.it1 - P.iw0 : 0;
+    MP_CUDA(h, h->tstate.ensure(((size_t)grid * (P.it1 - P.iw1) + nmod) * 4 + 64));
     const bool large = P.iend > P.it1;
     if (large) {
         MP_CUDA(h, h->rec.ensure((size_t)ntile * P.cap * 4));
@@ -1076,7 +1166,8 @@ int mp_planes_run(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, TileSu
     }
     a.cap = P.cap;
     a.planes = h->planes.as<u32>();
-    a.tstate = h->tstate.as<u32>();
+    a.tstate = h->tstate.as<u32>() + nmod;
+    a.imod = nmod ? h->tstate.as<u32>() : nullptr;
     PlaneScanArgs c;
     memset(&c, 0, sizeof c);
     c.g = g;
@@ -1124,16 +1215,24 @@ int mp_planes_run(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, TileSu
             plane_scatter_kernel<<<std::min(nblk, (s.k1 - s.k0 + 31) / 32), PS_THREADS, ssm, st>>>(s);
             MP_CUDA(h, cudaGetLastError());
         }
+        if (nmod) {
+            plane_imod_kernel<<<(nmod + 255) / 256, 256, 0, st>>>(a.q + P.iw0, a.magic + P.iw0, nmod, a.i0,
+                                                                  h->tstate.as<u32>());
+            MP_CUDA(h, cudaGetLastError());
+        }
         {
             ProfScope ps(h, PROF_TILE, st);
-            plane_tile_kernel<<<grid, P.threads, tsm, st>>>(a);
+            tile[tk]<<<grid, P.threads, tsm, st>>>(a);
         }
         MP_CUDA(h, cudaGetLastError());
         c.t0 = t0;
         c.nt = nt;
         ProfScope ps(h, PROF_FOLD, st);
-        if (bitmap32) plane_scan_kernel<true><<<nt, 32 * SCAN_WARPS, 0, st>>>(c);
-        else plane_scan_kernel<false><<<nt, 32 * SCAN_WARPS, 0, st>>>(c);
+        // two warps a stretch of 2^19 bits and more: a warp's first row and its summary cost several rows
+        // (at 2^20 bits 0.86 ms of scans a 2^34 integers, eight warps 0.96)
+        const u32 sth = g.tlog >= 19 ? 64 : 32 * SCAN_WARPS;
+        if (bitmap32) plane_scan_kernel<true><<<nt, sth, 0, st>>>(c);
+        else plane_scan_kernel<false><<<nt, sth, 0, st>>>(c);
         MP_CUDA(h, cudaGetLastError());
         if (emit_total) {
             plane_offsets_kernel<<<1, 1024, 0, st>>>(sums, t0, nt, off, emit_total);
