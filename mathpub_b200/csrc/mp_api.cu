@@ -247,13 +247,14 @@ int mp_primes_range(mp_handle *h, uint64_t lo, uint64_t hi, uint64_t *primes, si
     if (hi <= lo) return MP_OK;
     cudaStream_t st = h->stream;
     u64 n = 0;
-    // count first (cap 0), then emit into a device buffer of the exact size
-    MP_TRY(mp_sieve_emit_primes(h, lo, hi, nullptr, 0, &n, st));
+    if (!cap || !primes) {                               // counted only
+        MP_TRY(mp_sieve_emit_primes(h, lo, hi, nullptr, 0, &n, st));
+        *count = (size_t)n;
+        return MP_OK;
+    }
+    MP_TRY(mp_primes_to_device(h, lo, hi, h->ferm_p, &n, st));
     *count = (size_t)n;
     if (!n) return MP_OK;
-    MP_CUDA(h, h->ferm_p.ensure((size_t)n * 8));
-    u64 n2 = 0;
-    MP_TRY(mp_sieve_emit_primes(h, lo, hi, h->ferm_p.as<u64>(), n, &n2, st));
     const size_t m = std::min<size_t>(cap, (size_t)n);
     if (m && primes) MP_CUDA(h, cudaMemcpyAsync(primes, h->ferm_p.p, m * 8, cudaMemcpyDeviceToHost, st));
     MP_CUDA(h, cudaStreamSynchronize(st));
@@ -366,11 +367,8 @@ int mp_wieferich_range(mp_handle *h, uint64_t lo, uint64_t hi, mp_wief_stats *ou
     if (hi > (1ull << 63)) return mp_set_error(h, MP_ERANGE, "hi must be <= 2^63");
     cudaStream_t st = h->stream;
     u64 n = 0;
-    MP_TRY(mp_sieve_emit_primes(h, lo, hi, nullptr, 0, &n, st));
-    MP_CUDA(h, h->ferm_p.ensure((size_t)n * 8 + 8));
     MP_CUDA(h, h->stats_out.ensure(sizeof(mp_wief_stats) + 256));
-    u64 n2 = 0;
-    MP_TRY(mp_sieve_emit_primes(h, lo, hi, h->ferm_p.as<u64>(), n, &n2, st));
+    MP_TRY(mp_primes_to_device(h, lo, hi, h->ferm_p, &n, st));
     const int variant = ((hi - 1) >> 47 ? 1 : 0) | (h->tune.fermat_variant & 2);
     mp_wief_stats *ds = h->stats_out.as<mp_wief_stats>();
     MP_CUDA(h, cudaEventRecord(h->ev0, st));

@@ -976,13 +976,20 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS, 2) plane_scan_kernel(PlaneSca
     }
 }
 
-// the in-range primes of each stretch, in order, from place emit_off on (a thread's 32 blocks at a time)
-__global__ void __launch_bounds__(32 * SCAN_WARPS) plane_emit_kernel(PlaneScanArgs a)
+// the in-range primes of each stretch, in order, from place emit_off on.  A warp takes 32 words (1024
+// blocks of 30) at a time: the lanes put their primes as 16-bit offsets into the warp's part of shared
+// memory, and the warp writes them out in whole rows (36 M primes near 1e12: 0.13 ms, 0.44 with every
+// lane writing its own run)
+#define EMIT_WARPS 8
+#define EMIT_ROW 3328u                 // 30720 consecutive integers hold at most pi(30720) = 3313 primes above 5
+__global__ void __launch_bounds__(32 * EMIT_WARPS) plane_emit_kernel(PlaneScanArgs a)
 {
+    extern __shared__ __align__(16) u16 s_offs[];         // [EMIT_WARPS][EMIT_ROW]
     __shared__ Stretch S;
-    __shared__ u32 s_cnt[SCAN_WARPS];
+    __shared__ u32 s_cnt[EMIT_WARPS];
     const u32 tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const u32 t = a.t0 + blockIdx.x;
+    u16 *const out = s_offs + warp * EMIT_ROW;
     stretch_setup(S, a, t);
     u64 at = a.emit_off[t];
     if (S.A < 5)
@@ -991,7 +998,7 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS) plane_emit_kernel(PlaneScanAr
                 if (tid == 0 && at < a.emit_cap) a.emit[at] = x;
                 at++;
             }
-    for (u32 wr = S.w0; wr < S.w1; wr += 32 * SCAN_WARPS) {
+    for (u32 wr = S.w0; wr < S.w1; wr += 32 * EMIT_WARPS) {
         const u32 w = wr + tid;
         u32 p[8], c = 0;
 #pragma unroll
@@ -1005,29 +1012,32 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS) plane_emit_kernel(PlaneScanAr
             const u32 v = __shfl_up_sync(0xffffffffu, incl, d);
             if (lane >= (u32)d) incl += v;
         }
-        if (lane == 31) s_cnt[warp] = incl;
+        const u32 n = __shfl_sync(0xffffffffu, incl, 31);
+        if (lane == 0) s_cnt[warp] = n;
         __syncthreads();
         u32 before = 0, total = 0;
-        for (int i = 0; i < SCAN_WARPS; i++) {
+#pragma unroll
+        for (int i = 0; i < EMIT_WARPS; i++) {
             const u32 v = s_cnt[i];
             if (i < (int)warp) before += v;
             total += v;
         }
-        u64 pos = at + before + incl - c;
-        at += total;
-        u32 v[8];
+        u32 v[8], pos = incl - c;
         transpose_planes(v, p);
-        const u64 x0 = 30 * (a.i0 + (u64)w * 32);
 #pragma unroll
-        for (int b = 0; b < 32; b++) {
-            u32 y = (v[b >> 2] >> (8 * (b & 3))) & 0xffu;
-            while (y) {
+        for (int m = 0; m < 8; m++) {
+            const u32 x0 = 30 * (32 * lane + 4 * m);
+            for (u32 y = v[m]; y; y &= y - 1) {           // four blocks, a byte each
                 const u32 k = __ffs(y) - 1;
-                y &= y - 1;
-                if (pos < a.emit_cap) a.emit[pos] = x0 + 30 * b + pl_res(k);
+                if (pos < EMIT_ROW) out[pos] = (u16)(x0 + 30 * (k >> 3) + (__byte_perm(0x0d0b0701u, 0x1d171311u, k & 7) & 0xffu));
                 pos++;
             }
         }
+        __syncwarp();
+        const u64 x0 = 30 * (a.i0 + (u64)(wr + 32 * warp) * 32), to = at + before;
+        for (u32 i = lane; i < n; i += 32)
+            if (to + i < a.emit_cap) __stcs(a.emit + to + i, x0 + out[i]);
+        at += total;
         __syncthreads();
     }
 }
@@ -1236,7 +1246,11 @@ int mp_planes_run(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, TileSu
         MP_CUDA(h, cudaGetLastError());
         if (emit_total) {
             plane_offsets_kernel<<<1, 1024, 0, st>>>(sums, t0, nt, off, emit_total);
-            if (emit) plane_emit_kernel<<<nt, 32 * SCAN_WARPS, 0, st>>>(c);
+            if (emit) {
+                static bool emit_done[16] = {false};
+                MP_CUDA(h, raise_smem(plane_emit_kernel, emit_done, h->device, EMIT_WARPS * EMIT_ROW * 2));
+                plane_emit_kernel<<<nt, 32 * EMIT_WARPS, EMIT_WARPS * EMIT_ROW * 2, st>>>(c);
+            }
             MP_CUDA(h, cudaGetLastError());
         }
     }

@@ -128,13 +128,7 @@ int sieve_primes(mp_handle *w, u64 lo, u64 hi, u64 *n)
     std::shared_lock<std::shared_mutex> lk(g_tab);
     std::lock_guard<std::recursive_mutex> hl(w->mu);
     MP_CUDA(w, cudaSetDevice(w->device));
-    u64 c = 0, c2 = 0;
-    MP_TRY(mp_sieve_emit_primes(w, lo, hi, nullptr, 0, &c, w->stream));
-    if (!c) return MP_OK;
-    MP_CUDA(w, w->ferm_p.ensure((size_t)c * 8));
-    MP_TRY(mp_sieve_emit_primes(w, lo, hi, w->ferm_p.as<u64>(), c, &c2, w->stream));
-    *n = c;
-    return MP_OK;
+    return mp_primes_to_device(w, lo, hi, w->ferm_p, n, w->stream);
 }
 
 // copy the first n primes of the worker's device buffer to host memory
