@@ -35,9 +35,10 @@
 
 #define CS_K 131072u                          // values of k per class and segment
 #define CS_THREADS 256u
-#define CS_MAXG 64                            // pattern groups
-#define CS_SIEVE_LO 1024u                     // mp_chain_sieve: heads below this are checked one by one
-#define CS_PMAX_LIMIT 509u                    // pattern primes stay below CS_SIEVE_LO
+#define CS_MAXG 160                           // pattern groups
+#define CS_CU_MAXG 64                         // of them at most through cu_tables
+#define CS_SIEVE_LO 2048u                     // mp_chain_sieve: heads below this are checked one by one
+#define CS_PMAX_LIMIT 1021u                   // pattern primes stay below CS_SIEVE_LO
 #define CS_PERIOD_MAX (1u << 24)
 #define CS_MAXLEN (MP_CHAIN_MAX - 1)
 #define CS_NCNT (CU_MAXK + 2)                 // counters per shape: raw, after each round, final
@@ -279,11 +280,16 @@ __global__ void __launch_bounds__(CS_THREADS) cs_sieve_kernel(CsTables T, CsShap
     const u32 lane = threadIdx.x & 31;
     for (u32 c = 0; c < CS_CPB; c++) {
         if (jb * CS_CPB + c >= U.nj) break;                             // uniform
+        // word w of chunk i holds k = 32 (4 (thread + 256 i) + w) + b; chunks past the unit's last
+        // offset start dead, so that they load nothing
+        const u64 off0 = (u64)g * U.segsize + s_s0[c];
         u32 acc[4][4];
 #pragma unroll
-        for (u32 i = 0; i < 4; i++)
+        for (u32 i = 0; i < 4; i++) {
+            const u32 live = off0 + 128ull * (threadIdx.x + CS_THREADS * i) * U.W <= U.lim ? ~0u : 0u;
 #pragma unroll
-            for (u32 w = 0; w < 4; w++) acc[i][w] = ~0u;
+            for (u32 w = 0; w < 4; w++) acc[i][w] = live;
+        }
         for (u32 gi = 0; gi < T.ngroups; gi++) {
             const uint4 *pc = pat + s_chunk[c][gi] + threadIdx.x;
             const u32 bit = s_bit[c][gi], s = bit & 31;
@@ -294,8 +300,6 @@ __global__ void __launch_bounds__(CS_THREADS) cs_sieve_kernel(CsTables T, CsShap
             default: cs_and_group<3>(acc, pc, s); break;
             }
         }
-        // word w of chunk i holds k = 32 (4 (thread + 256 i) + w) + b
-        const u64 off0 = (u64)g * U.segsize + s_s0[c];
         if (off0 + (u64)(CS_K - 1) * U.W > U.lim) {                     // the unit's end: offsets <= lim only
 #pragma unroll
             for (u32 i = 0; i < 4; i++)
@@ -550,20 +554,23 @@ std::vector<u32> chain_offsets(u32 k, u32 shape)
 }
 
 // for the member offsets offs: the wheel (grown while W <= 3e7 and the classes number at most
-// 24,000), the pattern groups of the primes above it up to pattern_pmax (periods up to 2^24) and
+// 24,000; for a range of tier 2 while W <= 2^28 and they number at most 200,000), the pattern
+// groups of the primes above it up to pattern_pmax (periods up to 2^24) and
 // their patterns.  False when some prime leaves no admissible residue: then no p at or above
 // CS_SIEVE_LO has all its members prime.
 // the largest pattern prime for patterns of k members: the screen's work falls with the
 // survivors, each further prime q removing about k/q of them, while every group costs a window
 // read per live word; short patterns leave many survivors and gain from deeper patterns
-u32 pattern_pmax(u32 k)
+u32 pattern_pmax(u32 k, u32 tier)
 {
-    return (k >= 6 && k < 12) ? CS_PMAX_LIMIT : 199u;
+    return (k >= 6 && k < 9 && tier) ? CS_PMAX_LIMIT : (k >= 6 && k < 12) ? 509u : 199u;
 }
 
-bool make_plan(const std::vector<u32> &offs, CsPlan &P)
+bool make_plan(const std::vector<u32> &offs, u32 tier, CsPlan &P)
 {
-    const u32 pmax = pattern_pmax((u32)offs.size());
+    const bool wide = tier == 2;
+    const u32 pmax = pattern_pmax((u32)offs.size(), tier);
+    const u64 wmax = wide ? 1ull << 28 : 30000000ull, cmax = wide ? 200000 : 24000;
     static_assert(CS_PMAX_LIMIT < CS_SIEVE_LO, "members above CS_SIEVE_LO exceed every pattern prime");
     P.k = (u32)offs.size();
     P.offs = offs;
@@ -579,7 +586,7 @@ bool make_plan(const std::vector<u32> &offs, CsPlan &P)
             if (ok) adm.push_back(r);
         }
         if (adm.empty()) return false;
-        if (q > 2 && (W * q > 30000000ull || cls.size() * adm.size() > 24000)) break;
+        if (q > 2 && (W * q > wmax || cls.size() * adm.size() > cmax)) break;
         std::vector<u64> nc;                    // CRT: x = c (mod W), x = r (mod q)
         const u64 Wi = inv_mod(W % q, q);
         for (u64 c : cls)
@@ -713,8 +720,10 @@ __global__ void __launch_bounds__(128) cs_tuple128_kernel(const u64 *__restrict_
 struct ChainDev {
     u32 mode = 0, k = 0;
     std::vector<u32> key;                      // the member offsets the plan was built for
+    u32 tier = 0;                              // of the range's length (cs_prepare)
     bool ok = false;                           // false: no admissible p at or above CS_SIEVE_LO
     CsPlan plan;
+    ChainDev *other = nullptr;                 // the plan used before this one
     // the last chain list when the caller's arrays were too small, for the call that follows
     // with room for all of it (count first, then fill) so that the range is not sieved twice
     bool kept = false;
@@ -734,23 +743,51 @@ struct ChainDev {
 
 void mp_chain_free(mp_handle *h)
 {
-    if (!h->chain) return;
-    h->chain->release();
-    delete h->chain;
+    for (ChainDev *c = h->chain; c;) {
+        ChainDev *const o = c->other;
+        c->release();
+        delete c;
+        c = o;
+    }
     h->chain = nullptr;
 }
 
-// the handle's plan for (mode, offs), built and uploaded when it differs from the last one
-static int cs_prepare(mp_handle *h, u32 mode, const std::vector<u32> &offs)
+// Tiers of a range by its length.  From CS_WIDE_MIN on (3.6 segments of the wheel with 23) the wheel takes
+// one prime more: it strikes 23 by enumeration instead of by a pattern, 0.52 of the AND work at k = 11 and
+// 16 (1e15 integers at k = 11: 441 -> 302 ms, 2e15 at k = 16: 276 -> 180 ms); a
+// class costs its set-up however short its part of the range is.  From CS_DEEP_MIN on the patterns of 6
+// to 8 members go to 1021 instead of 509 (sextuplets of 2e12 integers 3.2 -> 2.5 ms; of 1e11 0.65 ->
+// 0.72 ms, so not below; to 2039 2.9 ms; 9 to 11 members to 1021: 302 -> 423 ms).
+#define CS_WIDE_MIN (6ull << 44)
+#define CS_DEEP_MIN (1ull << 39)
+
+// the handle's plan for (mode, offs) and a range of `len` integers, built and uploaded when it is none
+// of the last two
+static int cs_prepare(mp_handle *h, u32 mode, const std::vector<u32> &offs, u128t len)
 {
-    if (h->chain && h->chain->mode == mode && h->chain->key == offs) return MP_OK;
-    mp_chain_free(h);
+    const u32 tier = len >= CS_WIDE_MIN ? 2 : len >= CS_DEEP_MIN ? 1 : 0;
+    const auto fits = [&](const ChainDev *c) { return c && c->mode == mode && c->tier == tier && c->key == offs; };
+    if (fits(h->chain)) return MP_OK;
+    ChainDev *keep = h->chain;                             // it becomes the other one
+    if (keep && fits(keep->other)) {
+        h->chain = keep->other;
+        keep->other = nullptr;
+        h->chain->other = keep;
+        return MP_OK;
+    }
+    if (keep && keep->other) {
+        keep->other->release();
+        delete keep->other;
+        keep->other = nullptr;
+    }
     h->chain = new ChainDev();
+    h->chain->other = keep;
+    h->chain->tier = tier;
     ChainDev &D = *h->chain;
     D.mode = mode;
     D.k = (u32)offs.size();
     D.key = offs;
-    D.ok = make_plan(offs, D.plan);
+    D.ok = make_plan(offs, tier, D.plan);
     const CsPlan &P = D.plan;
     if (D.ok) {
         MP_CUDA(h, upload(D.ginfo, P.ginfo));
@@ -796,7 +833,12 @@ static int cs_sieve_range(mp_handle *h, ChainDev &D, u128t lo, u128t hi, cudaStr
     // for about 2^24 expected sieve survivors
     const double per_class = (double)CS_K * P.survive, target = 16777216.0;
     u32 useg = 1, ucls = A;
-    if (per_class * A <= target) useg = (u32)std::min<double>(256.0, std::floor(target / (per_class * A)));
+    // a unit spans at most 256 segments of the smaller wheel (below 2^50), so that a search for the first
+    // chain does not look further ahead with the larger one
+    const double span = D.tier == 2 ? 256.0 * CS_K * 9699690.0 : (double)(1ull << 50);
+    if (per_class * A <= target)
+        useg = (u32)std::max(1.0, std::min(std::min(256.0, std::floor(span / (double)segsize)),
+                                           std::floor(target / (per_class * A))));
     else ucls = (u32)std::max<double>(1.0, std::floor(target / per_class));
     u64 ucap = (u64)(1.25 * per_class * ucls * useg) + 65536;
     const CsTables T{D.ginfo.as<u32>(), D.q.as<u32>(), D.qinv.as<u32>(), D.crt.as<u32>(), (u32)(P.ginfo.size() / 4),
@@ -848,8 +890,7 @@ static int cs_collect(mp_handle *h, ChainDev &D, const u64 *list, const ull *nin
     MP_CUDA(h, cudaMemsetAsync(nres, 0, sizeof(ull), st));
     const u64 grid = std::max<u64>(1, std::min<u64>((expect + 127) / 128, (u64)h->sm_count * 16));
     // one-word arithmetic when every candidate, member and interloper of the list stays below
-    // 2^64 - 2^12: a unit spans at most 256 segments of 2^17 W < 2^17 3e7 integers (below 2^50),
-    // and members and extensions lie within 2^11 of their candidate
+    // 2^64 - 2^12: a unit spans less than 2^50 integers (one segment 2^17 W < 2^45), and members and extensions lie within 2^11 of their candidate
     if (base < ((u128t)1 << 64) - ((u128t)1 << 51))
         cs_verify64_kernel<<<(unsigned)grid, 128, 0, st>>>(list, nin, cap, (u64)base, D.k, D.mode, D.rh.as<u64>(),
                                                            D.rl.as<u32>(), nres);
@@ -881,7 +922,7 @@ static const u128t CS_HI128_MAX = (u128t)MP_CHAIN128_HI_MAX_W1 << 64 | MP_CHAIN1
 static int cs_chains(mp_handle *h, u128t lo, u128t hi, u32 k, u32 shape, std::vector<u128t> &H, std::vector<u32> &L)
 {
     cudaStream_t st = h->stream;
-    MP_TRY(cs_prepare(h, shape, chain_offsets(k, shape)));
+    MP_TRY(cs_prepare(h, shape, chain_offsets(k, shape), hi - lo));
     ChainDev &D = *h->chain;
     if (D.kept && D.kept_lo == lo && D.kept_hi == hi) {
         H.swap(D.kept_h);
@@ -963,7 +1004,7 @@ extern "C" int mp_chain_sieve128(mp_handle *h, const uint64_t lo[2], const uint6
 static int cs_first(mp_handle *h, u128t lo, u128t hi, u32 k, u32 shape, u128t *key, u128t *head, u32 *len)
 {
     cudaStream_t st = h->stream;
-    MP_TRY(cs_prepare(h, shape, chain_offsets(k, shape)));
+    MP_TRY(cs_prepare(h, shape, chain_offsets(k, shape), hi - lo));
     ChainDev &D = *h->chain;
     D.kept = false;
     std::vector<u128t> H;
@@ -1035,7 +1076,7 @@ static int cs_tuples(mp_handle *h, u128t lo, u128t hi, const uint32_t *offs, uin
                      uint64_t *cks)
 {
     cudaStream_t st = h->stream;
-    MP_TRY(cs_prepare(h, CS_MODE_TUPLE, std::vector<u32>(offs, offs + k)));
+    MP_TRY(cs_prepare(h, CS_MODE_TUPLE, std::vector<u32>(offs, offs + k), hi - lo));
     ChainDev &D = *h->chain;
     ull *acc = D.cnt.as<ull>() + CS_CNT_TUPLE;
     MP_CUDA(h, cudaMemsetAsync(acc, 0, 2 * sizeof(ull), st));
@@ -1163,7 +1204,7 @@ extern "C" int cu_tables(uint32_t ngroups, const uint32_t *ginfo, uint32_t nps, 
 {
     CuState &C = cu();
     std::lock_guard<std::mutex> lk(C.mu);
-    if (!C.init || !ngroups || ngroups > CS_MAXG || !nps || !ginfo || !q || !qinv || !crt) return -1;
+    if (!C.init || !ngroups || ngroups > CS_CU_MAXG || !nps || !ginfo || !q || !qinv || !crt) return -1;
     const std::vector<u32> gi(ginfo, ginfo + 4 * (size_t)ngroups), qq(q, q + nps), qi(qinv, qinv + nps),
         cr(crt, crt + nps);
     if (upload(C.ginfo, gi) || upload(C.q, qq) || upload(C.qinv, qi) || upload(C.crt, cr)) return -1;
