@@ -312,6 +312,7 @@ struct PlaneScatterArgs {
     const u64 *magic;
     u32 k0, k1;                       // the bucket primes
     u32 kc, run;                      // primes a warp takes from the queue at once: 32 below kc, then run
+    u32 parts, part;                  // below kc a unit is 32 primes over one of `parts` parts of `part` bits
     u32 *rec, *cnt;                   // [8 nb][cap], [8 nb] zeroed before the launch
     u32 cap;
     u32 *queue;                       // zeroed before the launch
@@ -391,7 +392,11 @@ __device__ __forceinline__ void plane_flush(const PlaneScatterArgs &a, u32 nt, u
 // of its multiples.  A thread holds one prime and the next hit of each plane, and files one hit per
 // plane and round; in plane order the eight starts follow from one remainder i0 mod q.  Warps take
 // runs of primes from a queue and hand them to the lanes that have none, so no lane waits for a
-// neighbour with more hits; the queue replaces bounds computed on the host for each range.
+// neighbour with more hits; the queue replaces bounds computed on the host for each range.  SMALL, for
+// waves with few units of work or few hits (2^16 integers at 9e17: 754 -> 260 us of scatter; 2^28 at
+// 1e12: 88 -> 42 us): units cover parts of the wave, a round looks for primes with hits up to eight
+// times, and primes far apart are first asked for any multiple at all.
+template <bool SMALL>
 __global__ void __launch_bounds__(PS_THREADS, PS_CTAS_PER_SM) plane_scatter_kernel(PlaneScatterArgs a)
 {
     extern __shared__ __align__(16) u32 ssm[];
@@ -413,44 +418,63 @@ __global__ void __launch_bounds__(PS_THREADS, PS_CTAS_PER_SM) plane_scatter_kern
         s_u[tid] = U;
         s_v[tid] = V;
     }
-    const u32 ni = a.ni, pt = a.pt, nb = a.nb, dense_q = ni / 2;
+    const u32 ni = a.ni, pt = a.pt, nb = a.nb, dense_q = (SMALL ? a.part : ni) / 2;
     u32 jj[8], q = 0;
     bool have = false;
-    u32 wk = 0, wend = 0;                                // the warp's run of primes
+    u32 wk = 0, wend = 0, wlo = 0, whi = ni;             // the warp's run of primes and part of the wave
+    u32 lim = 0;                                         // SMALL: the end of the lane's prime's part
     bool dry = false;                                    // the queue is empty
     __syncthreads();
     for (;;) {
-        // hand out primes to the lanes that have none; a prime without a hit is dropped on the spot, its
-        // lane tries again in the next round
-        const u32 need = __ballot_sync(0xffffffffu, !have);
-        if (need && wk >= wend && !dry) {
-            u32 c = 0;
-            if (lane == 0) c = atomicAdd(a.queue, 1u);
-            c = __shfl_sync(0xffffffffu, c, 0);
-            const u32 fine = (a.kc - a.k0) >> 5;         // kc - k0 is a multiple of 32
-            const u64 k = c < fine ? a.k0 + 32ull * c : a.kc + (u64)a.run * (c - fine);
-            wk = (u32)min(k, (u64)a.k1);
-            wend = min(wk + (c < fine ? 32u : a.run), a.k1);
-            dry = wk >= a.k1;
-        }
-        if (need && wk < wend) {
+        // hand out primes to the lanes that have none; a prime without a hit is dropped on the spot and
+        // its lane tries again, at most eight times a round
+        for (int tries = 0; tries < (SMALL ? 8 : 1); tries++) {
+            const u32 need = __ballot_sync(0xffffffffu, !have);
+            if (SMALL && tries && __popc(need) <= 16) break;
+            if (need && wk >= wend && !dry) {
+                u32 c = 0;
+                if (lane == 0) c = atomicAdd(a.queue, 1u);
+                c = __shfl_sync(0xffffffffu, c, 0);
+                const u32 parts = SMALL ? a.parts : 1u, fine = ((a.kc - a.k0) >> 5) * parts;   // kc - k0: whole 32s
+                const u32 pc = c / parts;
+                const u64 k = c < fine ? a.k0 + 32ull * pc : a.kc + (u64)a.run * (c - fine);
+                wk = (u32)min(k, (u64)a.k1);
+                wend = min(wk + (c < fine ? 32u : a.run), a.k1);
+                if (SMALL) {
+                    wlo = c < fine ? (c - pc * parts) * a.part : 0u;
+                    whi = c < fine ? min(wlo + a.part, ni) : ni;
+                }
+                dry = wk >= a.k1;
+            }
+            if (!need || wk >= wend) break;
             const u32 k = wk + __popc(need & lt);
             if (!have && k < wend) {
                 q = __ldg(a.q + k);
-                const u32 m = mp_mod_barrett(a.i0, q, __ldg(a.magic + k));
-                const u32 qa = q / 30u, c = q - 30u * qa;
-                const u64 U = s_u[c], V = s_v[c];
-                u32 jmin = 0xffffffffu;
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const u32 u = (u32)(U >> (8 * i)) & 0xffu, v = (u32)(V >> (8 * i)) & 0xffu;
-                    const u32 s = qa * u + v;
-                    u32 j = s - m + (s < m ? q : 0u);
-                    if (a.i0 <= qa && u == 1 && a.i0 + j == qa) j = q < ni ? j + q : ni;    // not q itself
-                    jj[i] = j;
-                    jmin = min(jmin, j);
+                const u64 magic = __ldg(a.magic + k), is = a.i0 + wlo;
+                bool hit = true;
+                if (SMALL && q / 32 > whi - wlo) {
+                    // far apart: most have no multiple, in a plane or not, in the part's integers
+                    const u32 r = mp_mod_barrett(30 * is, q, magic);
+                    hit = r == 0 || q - r < 30 * (whi - wlo);
                 }
-                have = jmin < ni;
+                if (hit) {
+                    const u32 m = mp_mod_barrett(is, q, magic);
+                    const u32 qa = q / 30u, c = q - 30u * qa;
+                    const u64 U = s_u[c], V = s_v[c];
+                    u32 jmin = 0xffffffffu;
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        const u32 u = (u32)(U >> (8 * i)) & 0xffu, v = (u32)(V >> (8 * i)) & 0xffu;
+                        const u32 s = qa * u + v;
+                        u32 j = s - m + (s < m ? q : 0u);
+                        if (is <= qa && u == 1 && is + j == qa) j = q < ni ? j + q : ni;    // not q itself
+                        if (SMALL) j = j < ni ? j + wlo : 0xffffffffu;   // from the wave's start
+                        jj[i] = j;
+                        jmin = min(jmin, j);
+                    }
+                    if (SMALL) lim = whi;
+                    have = jmin < (SMALL ? lim : ni);
+                }
             }
             wk = min(wk + (u32)__popc(need), wend);
         }
@@ -465,7 +489,7 @@ __global__ void __launch_bounds__(PS_THREADS, PS_CTAS_PER_SM) plane_scatter_kern
 #pragma unroll
         for (int i = 0; i < 8; i++) {
             const u32 j = jj[i];
-            const bool v = have && j < ni;
+            const bool v = have && j < (SMALL ? lim : ni);
             rec[i] = v ? __umulhi(j >> 10, a.blk_magic) * ((1u << PS_OFF_BITS) - pt) + (j + i * (nb << PS_OFF_BITS))
                        : PS_NONE;
             const u32 jn = v ? j + q : PS_NONE;
@@ -507,7 +531,7 @@ __global__ void __launch_bounds__(PS_THREADS, PS_CTAS_PER_SM) plane_scatter_kern
                 }
             }
         }
-        have = have && jmin < ni;
+        have = have && jmin < (SMALL ? lim : ni);
     }
     plane_flush(a, nt, stage, sorted, hist, gb, &s_fill, s_wsum);
 }
@@ -1122,6 +1146,8 @@ static int plan_planes(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, P
         P.iw0 = (u32)std::min<u64>(tb.count_le(89), P.iend);
         P.iw1 = std::max(P.iw0, (u32)std::min<u64>(tb.count_le(std::min<u32>(8192, P.pt / 64)), P.iend));
         P.it1 = std::max(P.iw1, (u32)std::min<u64>(tb.count_le((u64)P.pt * 3 / 2), P.iend));
+        // a few primes more a thread than a launch of their own
+        if (P.iend - P.it1 <= 16 * P.threads) P.it1 = P.iend;
         P.cap = 0;
         if (P.iend > P.it1) {
             // expected records of a tile: each bucket prime hits a block of pt bits pt / q times
@@ -1137,7 +1163,7 @@ static int plan_planes(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, P
 int mp_planes_run(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, TileSum *sums, u32 *bitmap32, u64 *emit,
                   u64 emit_cap, u64 *emit_total, cudaStream_t st)
 {
-    static bool tile_done[3][16] = {{false}}, scat_done[16] = {false};
+    static bool tile_done[3][16] = {{false}}, scat_done[2][16] = {{false}};
     PlanePlan P;
     MP_TRY(plan_planes(h, tb, g, P));
     int smem_max = 0;
@@ -1211,8 +1237,16 @@ int mp_planes_run(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, TileSu
             // runs of 32 primes where they take several rounds, then up to 512, so that the queue is no
             // bottleneck and no warp is left with a long run (measured: runs of 512 throughout, 6.4 ms
             // instead of 2.2 at 9e17, where a few warps held the smallest primes)
-            s.kc = s.k0 + (std::min(s.k1, std::max(s.k0, (u32)tb.count_le(s.ni / 4))) - s.k0 & ~31u);
-            s.run = std::max(32u, std::min(512u, (s.k1 - s.kc) / (nblk * (PS_THREADS / 32) * 8) & ~31u));
+            const bool far = tb.host[s.k1 - 1] / 32 > s.ni;                  // most primes have no hit
+            const u64 many = far ? 4ull * s.ni : s.ni / 4;                   // several rounds to here
+            s.kc = s.k0 + (std::min(s.k1, std::max(s.k0, (u32)tb.count_le(many))) - s.k0 & ~31u);
+            const u32 each = (s.k1 - s.kc) / (nblk * (PS_THREADS / 32));      // primes a warp
+            s.run = std::max(32u, std::min(512u, (far ? each / 2 : each / 8) & ~31u));
+            // with fewer of the former than eight per warp, each covers a part of the wave only, of four
+            // rounds or more: a wave of a small range waited for one warp's rounds
+            const u32 fine = (s.kc - s.k0) >> 5, rounds = s.ni / (P.pt + P.pt / 2) + 1;
+            s.parts = fine ? std::max(1u, std::min(8 * nblk * (PS_THREADS / 32) / fine, rounds / 4)) : 1u;
+            s.part = (s.ni + s.parts - 1) / s.parts;
             s.rec = h->rec.as<u32>(); s.cnt = h->reccnt.as<u32>(); s.cap = P.cap;
             s.queue = s.cnt + ntile;
             s.err = h->errflag.as<u32>();
@@ -1220,9 +1254,14 @@ int mp_planes_run(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, TileSu
             a.cnt = s.cnt;
             MP_CUDA(h, cudaMemsetAsync(s.cnt, 0, ((size_t)ntile + 1) * 4, st));
             const size_t ssm = ((size_t)2 * PS_STAGE + 2 * ntile) * 4;
-            MP_CUDA(h, raise_smem(plane_scatter_kernel, scat_done, h->device, smem_max - 4096));
+            // the form for small waves: parts, or primes so far apart that most have no multiple in the wave
+            const int sk = s.parts > 1 || far;
+            static void (*const scat[2])(PlaneScatterArgs) = {plane_scatter_kernel<false>, plane_scatter_kernel<true>};
+            MP_CUDA(h, raise_smem(scat[sk], scat_done[sk], h->device, smem_max - 4096));
             ProfScope ps(h, PROF_SCATTER, st);
-            plane_scatter_kernel<<<std::min(nblk, (s.k1 - s.k0 + 31) / 32), PS_THREADS, ssm, st>>>(s);
+            // a unit per CTA before a second one in any: a round's barriers are what a small wave waits for
+            const u32 units = fine * s.parts + (s.k1 - s.kc + s.run - 1) / s.run;
+            scat[sk]<<<std::min(nblk, units), PS_THREADS, ssm, st>>>(s);
             MP_CUDA(h, cudaGetLastError());
         }
         if (nmod) {

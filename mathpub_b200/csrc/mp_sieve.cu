@@ -2075,15 +2075,15 @@ static bool planes_form(const mp_handle *h, const mp_sieve_opts *o)
            h->tune.scatter_staged == 1 && h->tune.bucket_div == 1;
 }
 
-// the range and its stretches: 2^20 bits, fewer for ranges that would leave SMs without one, and no
-// more than a block
+// the range and its stretches: 2^20 bits, fewer for ranges that would leave SMs without one (one to two
+// an SM then, so that their scans are one round of CTAs), and no more than a block
 static int planes_geom(mp_handle *h, u64 lo, u64 hi, u32 block_log2, SieveGeom &g)
 {
     g.base = lo & ~1ull;
     g.limit = (hi - g.base) >> 1;
     g.nbx = (hi + MP_TAIL - g.base) >> 1;
     g.tlog = 20;
-    while (g.tlog > 14 && (g.nbx >> g.tlog) < 2 * (u64)h->sm_count) g.tlog--;
+    while (g.tlog > 15 && (g.nbx >> g.tlog) < (u64)h->sm_count) g.tlog--;
     if (block_log2 && g.tlog > block_log2 - 1) g.tlog = block_log2 - 1;
     const u64 n = (g.nbx + (1ull << g.tlog) - 1) >> g.tlog;
     if (n >= (1ull << 31)) return mp_set_error(h, MP_ERANGE, "range too long (%llu tiles)", (unsigned long long)n);
