@@ -138,8 +138,8 @@ __global__ void __launch_bounds__(256) bpsw_trial_kernel(const u64 *__restrict__
     }
 }
 
-// 2. base-2 test of the survivors; passers to `pass`
-__global__ void __launch_bounds__(256) bpsw_base2_kernel(const u64 *__restrict__ n, u32 total,
+// 2. base-2 test of the survivors; passers to `pass`.  64 to 512 threads a CTA (mp_tune_set)
+__global__ void __launch_bounds__(512) bpsw_base2_kernel(const u64 *__restrict__ n, u32 total,
                                                          const u32 *__restrict__ surv, const u32 *sctr,
                                                          u32 *__restrict__ pass, u32 *ctr)
 {
