@@ -48,6 +48,10 @@ HBM_FALLBACK_GBS = 6650.0
 TILE_TRAFFIC_BYTES = 597.9e6 + 297.7e6
 # the same for the persistent pipeline launch of one step (None until captured)
 PIPE_TRAFFIC_BYTES = None
+# the tile in bits and the bucket bound of the residue planes on the bench range, and the DRAM bytes of
+# one plane_tile_kernel launch there
+PLANE_SHAPE = (1720320, 2580469)
+PLANE_TRAFFIC_BYTES = None
 WORKLOAD = ("large-offset sieve [1e15, 1e15+2^34) per GPU, odd-only bitmap, sieving primes up to 31623048, "
             "wheel/pattern presieve 3..89, bucket sieve above the tile; outputs per-2^24-block pi, twins, "
             "6-tuples {0,4,6,10,12,16} with checksum, max gap + start, per-2^20 FNV-1a bitmap hashes")
@@ -232,9 +236,9 @@ def run_ours(args):
     def max_over_ranks(x):
         return shard.max_over_ranks(x, device=dev)
 
-    # the measured autotuner picks the tile geometry at this height (and the Fermat variant)
+    # the measured autotuner picks the sieve's form and geometry at this height (and the Fermat variant)
     tune_report = e.autotune(LO) if args.autotune else "off"
-    # warm-up (builds the prime tables and captures the graph on the first call)
+    # warm-up (builds the prime tables and captures the graph)
     for _ in range(args.warmup):
         sieve_dev()
     barrier()
@@ -359,6 +363,11 @@ def run_ours(args):
         primes = e.primes_range(3, int(np.sqrt(float(hi + (1 << 16)))) + 2)
         tile_bits = 1 << 20
         import re
+        # residue planes (the default form): 8 planes of 1 bit per 30 integers, their tile and bucket
+        # bound from the report, or the bench range's own without one
+        odd_only = "sieve choice: tile" in tune_report
+        m = re.search(r"residue planes, (\d+)-bit tiles, buckets above (\d+)", tune_report)
+        plane_tile, plane_bucket = (int(m.group(1)), int(m.group(2))) if m else PLANE_SHAPE
         m = re.search(r"sieve choice: tile 2\^(\d+)", tune_report)
         if m:
             tile_bits = 1 << int(m.group(1))
@@ -366,9 +375,21 @@ def run_ours(args):
         bucket_div = int(m.group(1)) if m else 1
         ntiles = -(-((hi + (1 << 16) - lo) // 2) // tile_bits)
         staged = "binned scatter" not in tune_report.split("sieve choice")[-1]
-        marks_small, marks_large = algorithmic_work(primes, lo, hi, tile_bits // bucket_div, staged)
+        if odd_only:
+            marks_small, marks_large = algorithmic_work(primes, lo, hi, tile_bits // bucket_div, staged)
         pipe_launches, pipe_ms = prof.get("pipeline", (0, 0.0))
-        if pipe_launches:
+        bucket_above = tile_bits // bucket_div
+        if not odd_only:
+            # the planes' primes all mark the k coprime to 30, one per plane and multiple; a tile's launch
+            # reads the bucket records and writes the planes
+            marks_small, marks_large = algorithmic_work(primes, lo, hi, plane_bucket, staged=False)
+            bucket_above = plane_bucket
+            kname, klaunches, kms = f"plane_tile_kernel ({plane_tile}-bit tiles)", tile_launches, tile_ms
+            kbytes = (marks_large * 4 + 8 * ((hi + (1 << 16) - lo) // 30) / 8) / max(tile_launches, 1)
+            ktraffic = PLANE_TRAFFIC_BYTES
+            knote = ("bytes = bucket records read (4 B per large-prime hit) + residue planes written; the kernel is "
+                     "bound by shared-memory atomics, see roofline_smem")
+        elif pipe_launches:
             # one persistent launch per step runs the scatter and the tiles: its bytes are the
             # bucket records written and read back (4 B each way) and the bitmap written
             kname, klaunches, kms = "sieve_pipeline_kernel", pipe_launches, pipe_ms
@@ -409,7 +430,7 @@ def run_ours(args):
                          "frac": achieved / hbm, "traffic": ktraffic, "kernel": kname,
                          "peak_source": f"{hbm_src} (MEASURED_PEAKS.json hbm_gbs)" if hbm_src == "measured" else "fallback",
                          "algorithmic_bytes_per_launch": kbytes, "avg_launch_ms": tile_avg_s * 1e3,
-                         "bucket_threshold": tile_bits // bucket_div, "note": knote},
+                         "bucket_threshold": bucket_above, "note": knote},
             "roofline_smem": {"bound": "smem_atomics", "achieved": smem_marks_rate,
                               "peak": peaks["smem_atomic_conflict_free"], "unit": "atomic ops/s",
                               "frac": smem_marks_rate / peaks["smem_atomic_conflict_free"],
@@ -432,7 +453,8 @@ def run_ours(args):
                          "note": "achieved = Montgomery products counted exactly from the inputs (base-2 ladders of "
                                  "the trial-division survivors, Lucas ladders of the primes; chain squarings and "
                                  "set-up left out: a lower bound) x 32-bit multiply instructions per product / "
-                                 "kernel time; peak = the 32-bit IMAD rate measured in this run"}),
+                                 "kernel time; a squaring of the batched ladders takes fewer instructions than a "
+                                 "product, so frac can pass 1; peak = the 32-bit IMAD rate measured in this run"}),
                      "workload": "2^26 seeded odd u64 (60% uniform [2^40,2^64), 30% p*q near 2^62, "
                                  "10% (k+1)(2k+1) / Chernick), 4096 lists, log-uniform lengths"},
             "config1": config1,
@@ -565,7 +587,8 @@ def run_fermat(e, world, rank, dev, imad_peak):
     roof = imad_roofline(products * IMAD_PER_PRODUCT_FERMAT_K3, kms, imad_peak, {
         "products": products, "imad_per_product": IMAD_PER_PRODUCT_FERMAT_K3,
         "note": "achieved = (bitlen(p - 1) + 1) three-limb Montgomery products per prime x 39 32-bit multiply "
-                "instructions per product / time of the quotient and statistics kernels"})
+                "instructions per product / time of the quotient and statistics kernels; the ladder's squarings take "
+                "fewer and its first bits none, so frac can pass 1"})
     return {"workload": "base-2 Fermat quotients of every prime in [1e12, 1e12+4e9) (per rank), 3-limb Montgomery",
             "tests": r["tests"], "tests_per_s": r["tests"] / (kms / 1e3), "kernel_ms": kms, "roofline": roof,
             "e2e_tests_per_s": r["tests"] / wall, "e2e_ms": wall * 1e3, "near": r["near"], "flt": r["flt"],

@@ -1160,6 +1160,15 @@ static int plan_planes(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, P
     }
 }
 
+int mp_planes_shape(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, u32 *tile_bits, u32 *bucket_above)
+{
+    PlanePlan P;
+    MP_TRY(plan_planes(h, tb, g, P));
+    *tile_bits = P.pt;
+    *bucket_above = P.it1 ? tb.host[P.it1 - 1] : 0;
+    return MP_OK;
+}
+
 int mp_planes_run(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, TileSum *sums, u32 *bitmap32, u64 *emit,
                   u64 emit_cap, u64 *emit_total, cudaStream_t st)
 {

@@ -2077,7 +2077,7 @@ static bool planes_form(const mp_handle *h, const mp_sieve_opts *o)
 
 // the range and its stretches: 2^20 bits, fewer for ranges that would leave SMs without one (one to two
 // an SM then, so that their scans are one round of CTAs), and no more than a block
-static int planes_geom(mp_handle *h, u64 lo, u64 hi, u32 block_log2, SieveGeom &g)
+int mp_planes_geom(mp_handle *h, u64 lo, u64 hi, u32 block_log2, SieveGeom &g)
 {
     g.base = lo & ~1ull;
     g.limit = (hi - g.base) >> 1;
@@ -2112,7 +2112,7 @@ int mp_sieve_run(mp_handle *h, u64 lo, u64 hi, const mp_sieve_opts *o, mp_range_
     MP_TRY(mp_tables_ensure(h, mp_isqrt64(top - 1)));
     SievePlan P;
     const bool planes = mode == MP_MODE_BATCHED && planes_form(h, o);
-    if (planes) MP_TRY(planes_geom(h, lo, hi, block_log2, P.g));
+    if (planes) MP_TRY(mp_planes_geom(h, lo, hi, block_log2, P.g));
     else MP_TRY(plan_sieve(h, *h->tab, lo, hi, tlog, nth, P));
     tlog = P.g.tlog;
     MP_CUDA(h, h->tilesum.ensure((size_t)P.g.ntiles * sizeof(TileSum)));
@@ -2185,7 +2185,7 @@ int mp_sieve_emit_primes(mp_handle *h, u64 lo, u64 hi, u64 *d_primes, u64 cap, u
     if (planes_form(h, nullptr)) {
         // counted and written in one pass: the primes past cap are counted only
         SieveGeom g;
-        MP_TRY(planes_geom(h, lo, hi, 0, g));
+        MP_TRY(mp_planes_geom(h, lo, hi, 0, g));
         MP_CUDA(h, h->tilesum.ensure((size_t)g.ntiles * sizeof(TileSum)));
         MP_CUDA(h, h->small_out.ensure(256));
         u64 *total = h->small_out.as<u64>() + 24;

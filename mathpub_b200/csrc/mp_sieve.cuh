@@ -103,3 +103,8 @@ __device__ __forceinline__ u32 bits_mask(u64 start, u64 bound)
 // number goes to *emit_total, a device word, as always)
 int mp_planes_run(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, TileSum *sums, u32 *bitmap32, u64 *emit,
                   u64 emit_cap, u64 *emit_total, cudaStream_t st);
+
+// the stretches of a range in that form; and the tile of a plane in bits, with the bound above which
+// its primes go through the bucket scatter
+int mp_planes_geom(mp_handle *h, u64 lo, u64 hi, u32 block_log2, SieveGeom &g);
+int mp_planes_shape(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, u32 *tile_bits, u32 *bucket_above);

@@ -1,11 +1,12 @@
-// mp_tune.cu -- the measured autotuner: times the sieve tile geometry (bits per tile x
-// threads per CTA), the bucket scatter's form, the bucket threshold, the batched form
-// (persistent pipeline or wave loop), the Fermat kernel variants (limbs fixed by p, one or two
-// primes per thread) and the threads per CTA of the batched base-2 test
-// on the device with CUDA events, and keeps the fastest per handle.  The reference
-// chooses its wheel and chunk by a fitted cost model (auto_wheel / auto_chunk,
+// mp_tune.cu -- the measured autotuner: times the sieve's forms (residue planes, which size
+// themselves, and the odd-only tiles by bits per tile x threads per CTA, then their bucket
+// scatter's form, bucket threshold, and persistent pipeline or wave loop), the Fermat kernel
+// variants (limbs fixed by p, one or two primes per thread) and the threads per CTA of the
+// batched base-2 test on the device with CUDA events, and keeps the fastest per handle.  The
+// reference chooses its wheel and chunk by a fitted cost model (auto_wheel / auto_chunk,
 // A350826/a350826.c:1976-2015); here the candidates are timed instead.
 #include "mp_common.cuh"
+#include "mp_sieve.cuh"
 #include <algorithm>
 
 static int time_sieve(mp_handle *h, u64 lo, u64 hi, u32 tlog, u32 nth, mp_range_stats *d_out, float *ms)
@@ -25,38 +26,18 @@ static int time_sieve(mp_handle *h, u64 lo, u64 hi, u32 tlog, u32 nth, mp_range_
     return MP_OK;
 }
 
-extern "C" int mp_autotune(mp_handle *h, uint64_t lo, char *report, size_t cap)
+// a choice replaces the default only when it is more than 2% faster, so that timing noise between
+// near-equal forms does not decide
+static const float margin = 1.02f;
+
+// pin the odd-only tiles' fastest geometry, then their other knobs at it
+static int tune_tiles(mp_handle *h, u64 lo, u64 span, u32 bt, u32 bn, float best, float dflt, mp_range_stats *d_out,
+                      std::string &rep)
 {
-    if (!h) return MP_EINVAL;
-    std::lock_guard<std::recursive_mutex> lk(h->mu);
-    MP_CUDA(h, cudaSetDevice(h->device));
-    std::string rep;
     char line[160];
-    // sieve: a range of 2^34 integers at height lo (several waves, as in long scans); a choice
-    // replaces the default only when it is more than 2% faster, so that timing noise between
-    // near-equal forms does not decide
-    const u64 span = 1ull << 34;
-    const float margin = 1.02f;
-    if (lo > MP_HI_MAX - span) lo = MP_HI_MAX - span;
-    MP_CUDA(h, h->small_out.ensure(4096));
-    mp_range_stats *d_out = (mp_range_stats *)h->small_out.p;
-    float best = 1e30f, dflt = 1e30f;
-    u32 bt = 20, bn = 1024;
-    static const u32 tl[3] = {18, 19, 20}, th[3] = {256, 512, 1024};
-    for (u32 a : tl)
-        for (u32 b : th) {
-            float ms = 0;
-            const int r = time_sieve(h, lo, lo + span, a, b, d_out, &ms);
-            if (r != MP_OK) return r;
-            snprintf(line, sizeof line, "sieve tile 2^%u x %u threads: %.3f ms / 2^34\n", a, b, ms / 3);
-            rep += line;
-            if (ms < best) { best = ms; bt = a; bn = b; }
-            if (a == 20 && b == 1024) dflt = ms;
-        }
     if (dflt <= best * margin) { bt = 20; bn = 1024; }
     h->tune.sieve_tile_log2 = (int)bt;
     h->tune.sieve_threads = (int)bn;
-    h->tune.tuned_at = lo;
     h->tune_gen++;
     // one knob at a time at that geometry, on the same range, the first value the default:
     //   the bucket scatter's form: staged (three CTAs per SM, a sorted stage) or binned (one
@@ -92,6 +73,53 @@ extern "C" int mp_autotune(mp_handle *h, uint64_t lo, char *report, size_t cap)
              bn, h->tune.scatter_staged ? "staged" : "binned", h->tune.bucket_div,
              (h->tune.no_pipeline || h->tune.scatter_staged) ? "wave loop" : "pipeline");
     rep += line;
+    return MP_OK;
+}
+
+extern "C" int mp_autotune(mp_handle *h, uint64_t lo, char *report, size_t cap)
+{
+    if (!h) return MP_EINVAL;
+    std::lock_guard<std::recursive_mutex> lk(h->mu);
+    MP_CUDA(h, cudaSetDevice(h->device));
+    std::string rep;
+    char line[160];
+    // sieve: a range of 2^34 integers at height lo (several waves, as in long scans)
+    const u64 span = 1ull << 34;
+    if (lo > MP_HI_MAX - span) lo = MP_HI_MAX - span;
+    MP_CUDA(h, h->small_out.ensure(4096));
+    mp_range_stats *d_out = (mp_range_stats *)h->small_out.p;
+    // the residue planes, which a call takes unless a geometry or knob of the odd-only tiles is pinned,
+    // against every geometry of those ([1e15, +2^34) without hashes: 6.2 ms against 9.8 for the best)
+    h->tune.sieve_tile_log2 = h->tune.sieve_threads = 0;
+    h->tune.scatter_staged = h->tune.bucket_div = 1;
+    h->tune_gen++;
+    float planes = 0, best = 1e30f, dflt = 1e30f;
+    MP_TRY(time_sieve(h, lo, lo + span, 0, 0, d_out, &planes));
+    snprintf(line, sizeof line, "sieve residue planes: %.3f ms / 2^34\n", planes / 3);
+    rep += line;
+    u32 bt = 20, bn = 1024;
+    static const u32 tl[3] = {18, 19, 20}, th[3] = {256, 512, 1024};
+    for (u32 a : tl)
+        for (u32 b : th) {
+            float ms = 0;
+            const int r = time_sieve(h, lo, lo + span, a, b, d_out, &ms);
+            if (r != MP_OK) return r;
+            snprintf(line, sizeof line, "sieve tile 2^%u x %u threads: %.3f ms / 2^34\n", a, b, ms / 3);
+            rep += line;
+            if (ms < best) { best = ms; bt = a; bn = b; }
+            if (a == 20 && b == 1024) dflt = ms;
+        }
+    h->tune.tuned_at = lo;
+    if (planes <= best * margin) {
+        u32 pt = 0, q = 0;
+        SieveGeom g;
+        MP_TRY(mp_planes_geom(h, lo, lo + span, 0, g));
+        MP_TRY(mp_planes_shape(h, *h->tab, g, &pt, &q));
+        snprintf(line, sizeof line, "sieve choice: residue planes, %u-bit tiles, buckets above %u\n", pt, q);
+        rep += line;
+    } else {
+        MP_TRY(tune_tiles(h, lo, span, bt, bn, best, dflt, d_out, rep));
+    }
     // Fermat: 2^20 primes near max(lo, 1e12), one vs two per thread
     u64 plo = std::max<u64>(lo, 1000000000000ull);
     if (plo > (1ull << 62)) plo = 1ull << 40;
