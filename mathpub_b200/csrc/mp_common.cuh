@@ -124,12 +124,13 @@ struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;
     u64 *gen = nullptr;
-    cudaError_t ensure(size_t need)
+    // spare: bytes more where it has to grow, for a size that differs a little from call to call
+    cudaError_t ensure(size_t need, size_t spare = 0)
     {
         if (need <= bytes && p) return cudaSuccess;
         if (p) { cudaFree(p); p = nullptr; bytes = 0; }
         if (gen) (*gen)++;
-        size_t b = need < 256 ? 256 : need;
+        size_t b = (need < 256 ? 256 : need) + spare;
         cudaError_t e = cudaMalloc(&p, b);
         if (e == cudaSuccess) bytes = b;
         return e;

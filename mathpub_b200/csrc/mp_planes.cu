@@ -1185,13 +1185,20 @@ int mp_planes_run(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, TileSu
     int occ = 0;
     MP_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, tile[tk], (int)P.threads, tsm));
     const u32 grid = (u32)std::min<u64>(ntile, (u64)h->sm_count * (u32)std::max(occ, 1));
-    MP_CUDA(h, h->planes.ensure(((size_t)ntile * nw + 64) * 4));
+    // The buffers follow the range's length and, a little, its height; a growth frees the old one, which
+    // waits for the device ([1e12 + x, +2^30) for growing x: 1.1 ms instead of 0.27).  So they grow with
+    // something to spare; a third for the threads' state, which is largest below the longest waves
+    // (tiles of less than half an SM's shared memory run two to an SM).
+    const size_t spare = 32u << 20, psize = ((size_t)ntile * nw + 64) * 4;
+    MP_CUDA(h, h->planes.ensure(psize, psize / 16 + spare));
     const u32 nmod = P.it1 - P.iw0 >= PL_IMOD_MIN ? P.it1 - P.iw0 : 0;
-    MP_CUDA(h, h->tstate.ensure(((size_t)grid * (P.it1 - P.iw1) + nmod) * 4 + 64));
+    const size_t tsize = ((size_t)grid * (P.it1 - P.iw1) + nmod) * 4 + 64;
+    MP_CUDA(h, h->tstate.ensure(tsize, tsize / 3 + spare / 4));
     const bool large = P.iend > P.it1;
     if (large) {
-        MP_CUDA(h, h->rec.ensure((size_t)ntile * P.cap * 4));
-        MP_CUDA(h, h->reccnt.ensure(((size_t)ntile + 1) * 4));
+        const size_t rsize = (size_t)ntile * P.cap * 4;
+        MP_CUDA(h, h->rec.ensure(rsize, rsize / 16 + spare));
+        MP_CUDA(h, h->reccnt.ensure(((size_t)ntile + 1) * 4, 16384));
     }
     PlaneTileArgs a;
     memset(&a, 0, sizeof a);
@@ -1224,7 +1231,7 @@ int mp_planes_run(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, TileSu
     c.emit_cap = emit_cap;
     u64 *off = nullptr;
     if (emit_total) {
-        MP_CUDA(h, h->emit_off.ensure((size_t)g.ntiles * 8 + 64));
+        MP_CUDA(h, h->emit_off.ensure((size_t)g.ntiles * 8 + 64, 65536));
         off = h->emit_off.as<u64>();
         c.emit_off = off;
         MP_CUDA(h, cudaMemsetAsync(emit_total, 0, 8, st));

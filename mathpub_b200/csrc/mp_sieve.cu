@@ -2015,7 +2015,7 @@ int mp_tables_ensure(mp_handle *h, u64 limit)
     MP_TRY(plan_sieve(h, h->boot, lo, hi, 20, 1024, P));
     // the tail is not needed for a prime list, but plan_sieve adds it; primes beyond hi are
     // not emitted (limit bits)
-    MP_CUDA(h, h->tilesum.ensure((size_t)P.g.ntiles * sizeof(TileSum)));
+    MP_CUDA(h, h->tilesum.ensure((size_t)P.g.ntiles * sizeof(TileSum), 65536));
     MP_CUDA(h, h->blockacc.ensure((size_t)P.g.ntiles * 8 + 16));
     TileArgs a;
     fill_tile_args(h, h->boot, P, a);
@@ -2115,7 +2115,7 @@ int mp_sieve_run(mp_handle *h, u64 lo, u64 hi, const mp_sieve_opts *o, mp_range_
     if (planes) MP_TRY(mp_planes_geom(h, lo, hi, block_log2, P.g));
     else MP_TRY(plan_sieve(h, *h->tab, lo, hi, tlog, nth, P));
     tlog = P.g.tlog;
-    MP_CUDA(h, h->tilesum.ensure((size_t)P.g.ntiles * sizeof(TileSum)));
+    MP_CUDA(h, h->tilesum.ensure((size_t)P.g.ntiles * sizeof(TileSum), 65536));
     // bitmap: the caller's, or scratch when only hashes are wanted
     const u64 nwords64 = (P.g.limit + 63) >> 6;
     u32 *bm = (u32 *)d_bitmap;
@@ -2147,7 +2147,7 @@ int mp_sieve_run(mp_handle *h, u64 lo, u64 hi, const mp_sieve_opts *o, mp_range_
     }
     const u64 nbe = (P.g.ntiles + tpb - 1) / tpb;
     if (nbe > (1ull << 26)) return mp_set_error(h, MP_ERANGE, "too many blocks");
-    MP_CUDA(h, h->blockacc.ensure((size_t)nbe * sizeof(Part)));
+    MP_CUDA(h, h->blockacc.ensure((size_t)nbe * sizeof(Part), 65536));
     FoldArgs f;
     f.base = P.g.base; f.limit = P.g.limit; f.lo = lo; f.hi = hi;
     f.sums = h->tilesum.as<TileSum>(); f.ntiles = P.g.ntiles; f.tpb = tpb;
@@ -2205,7 +2205,7 @@ int mp_sieve_emit_primes(mp_handle *h, u64 lo, u64 hi, u64 *d_primes, u64 cap, u
     }
     SievePlan P;
     MP_TRY(plan_sieve(h, *h->tab, lo, hi, tlog, nth, P));
-    MP_CUDA(h, h->tilesum.ensure((size_t)P.g.ntiles * sizeof(TileSum)));
+    MP_CUDA(h, h->tilesum.ensure((size_t)P.g.ntiles * sizeof(TileSum), 65536));
     MP_CUDA(h, h->blockacc.ensure((size_t)P.g.ntiles * 8 + 16));
     TileArgs a;
     fill_tile_args(h, *h->tab, P, a);
