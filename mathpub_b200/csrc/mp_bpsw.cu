@@ -25,14 +25,18 @@
 //            division and the base-2 test left batches partly filled (25 of 32 lanes active) and,
 //            at 2^24 candidates, 2.3 chunks a warp: 1.13 ms for the two
 //            phases that take 1.01 ms now (1.38 ms before the windowed ladder).
-//   few      up to BPSW_FEW candidates: one launch with every phase inline, a warp per 32
-//            candidates, since latency is all that counts there
+//   few      up to BPSW_FEW candidates: one launch whose warps take the phases of a candidate at the
+//            same time, since latency is all that counts there
 #include "mp_mont64.cuh"
 #include <algorithm>
 
-// up to this many candidates a batch runs in one launch (a warp per SM subpartition and more warps
-// idle than busy): 100 candidates 28 us of kernel against 57 in the launches of the batched form
-#define BPSW_FEW 8192
+// Up to BPSW_FEW candidates a batch runs in one launch (a whole call with host copies, batched form
+// against this: 100 candidates 83 and 51 us, 4000 89 and 66, 16000 118 and 86, 24000 122 and 102; the
+// former needs no Lucas tests of composites, so that it is taken well before they meet), of 8
+// candidates a CTA up to BPSW_VERY_FEW (8 against 32 a CTA: 1000 candidates 53 and 59 us, 2000 57 and
+// 65, 4000 67 and 66).
+#define BPSW_FEW 16384
+#define BPSW_VERY_FEW 2048
 
 #define TD_N 30            // odd primes 3..127
 #define TD_NG 6            // in six groups whose products are below 2^32
@@ -81,6 +85,63 @@ __global__ void __launch_bounds__(256) bpsw_plain_kernel(const u64 *__restrict__
     if (i < len) v = bpsw_full(__ldg(n + i));
     const u32 b = __ballot_sync(0xffffffffu, v);
     if ((threadIdx.x & 31) == 0 && i < len) bits[i >> 5] = b;
+}
+
+// ---- few candidates ----
+// G candidates of one list per CTA, whose four warps take the phases at the same time: the base-2 test
+// below 2^63 and above, and the Lucas test for D = 5 and for any other D, each after its own search for
+// D (W = 32 / G lanes a candidate try W values of D at once).  Latency is all that counts, so the Lucas
+// ladders of composites, which the phases in turn would save, cost nothing (100 candidates: 21 us of
+// kernel, 28 with a thread per candidate and the phases in turn).
+template <int G>
+__global__ void __launch_bounds__(128) bpsw_few_kernel(const u64 *__restrict__ n, u32 total, u32 *__restrict__ bits)
+{
+    constexpr u32 W = 32 / G;
+    __shared__ u32 s_pass[4];
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % W, i = blockIdx.x * G + lane / W;
+    const u64 x = i < total ? __ldg(n + i) : 0;
+    const int td = td_verdict(x);
+    const bool open = td < 0 && x != ~0ull;                              // 3 | 2^64 - 1
+    bool v = false;
+    if (warp < 2) {
+        if (open && sub == 0 && x >> 63 == warp) v = warp ? spsp2<SP_WIDE>(x) : spsp2<SP_MID>(x);
+    } else {
+        // selfridge_d, W tries a round: the first D with (D/n) <= 0 decides
+        i32 D = 0;
+        bool more = open;
+        for (int k0 = 0; k0 < 2048 && __any_sync(0xffffffffu, more); k0 += W) {
+            const int k = k0 + (int)sub;
+            const i32 a = 5 + 2 * k, d = (k & 1) ? -a : a;
+            const int j = more ? jacobi_dn(d, x) : 1;
+            const u32 neg = __ballot_sync(0xffffffffu, more && j < 0), zero = __ballot_sync(0xffffffffu, more && j == 0);
+            const u32 own = (W == 32 ? 0xffffffffu : (1u << (W & 31)) - 1) << (lane - sub), ev = (neg | zero) & own;
+            const u32 first = ev ? __ffs((int)ev) - 1 : lane;
+            const i32 df = __shfl_sync(0xffffffffu, d, (int)first);
+            if (more && ev) {
+                more = false;
+                D = neg >> first & 1 ? df : 0;
+            } else if (more && k0 <= 23 && k0 + (int)W > 23 && is_square64(x)) {
+                more = false;
+            }
+        }
+        if (D && sub == 0 && (D == 5) == (warp == 2)) {
+            const Mod64 M = mm_setup(x);
+            v = warp == 2 ? lucas_strong_d5(M) : lucas_strong(M, D);
+        }
+    }
+    __syncwarp();
+    const u32 m = __ballot_sync(0xffffffffu, v);
+    if (lane == 0) s_pass[warp] = m;
+    __syncthreads();
+    if (warp == 0) {
+        const u32 pass = (s_pass[0] | s_pass[1]) & (s_pass[2] | s_pass[3]), at = lane * W & 31;
+        const int tj = __shfl_sync(0xffffffffu, td, (int)at);
+        const u32 b = __ballot_sync(0xffffffffu, lane < G && (tj == 1 || (pass >> at & 1)));
+        if (lane == 0) {
+            if (G == 32) bits[blockIdx.x] = b;
+            else ((u8 *)bits)[blockIdx.x] = (u8)b;
+        }
+    }
 }
 
 // ---- batched form ----
@@ -309,7 +370,9 @@ int mp_bpsw_run(mp_handle *h, const u64 *d_n, const u64 *offs, const u32 *lens, 
     if (!total) return MP_OK;
     if (total <= BPSW_FEW) {
         ProfScope ps(h, PROF_BPSW_BATCHED, st);
-        bpsw_plain_kernel<<<(unsigned)((total + 31) / 32), 32, 0, st>>>(d_n, (u32)total, d_bits);
+        const unsigned words = (unsigned)((total + 31) / 32);
+        if (total <= BPSW_VERY_FEW) bpsw_few_kernel<8><<<4 * words, 128, 0, st>>>(d_n, (u32)total, d_bits);
+        else bpsw_few_kernel<32><<<words, 128, 0, st>>>(d_n, (u32)total, d_bits);
         MP_CUDA(h, cudaGetLastError());
         return MP_OK;
     }
