@@ -88,12 +88,13 @@ typedef struct {
 
 typedef mp_range_stats mp_block_stats;
 
-/* MP_MODE_BATCHED: the range in waves of tiles; per wave a bucket scatter for the large
- *   primes, then a tile launch in which each CTA sieves a contiguous run of tiles and carries
- *   the state of its sparse primes from tile to tile; the whole call is captured once as a
- *   CUDA graph and replayed.  With the binned scatter (mp_tune_set) and no
+/* MP_MODE_BATCHED: the range in waves, in eight residue planes mod 30; per wave a bucket scatter for the
+ *   large primes, a tile launch in which each CTA sieves a contiguous run of tiles and carries
+ *   the state of its sparse primes from tile to tile, and a scan of the planes; a call that
+ *   repeats is captured as a CUDA graph and replayed.  With a pinned geometry or knob of the
+ *   odd-only tiles (below, mp_tune_set) the waves run in those; with their binned scatter and no
  *   MP_TUNE_NO_PIPELINE, one persistent launch runs every wave's scatter and tile work from a
- *   device queue instead.
+ *   device queue.
  * MP_MODE_PLAIN: the reference's per-segment launch loop on a full grid: one launch per group
  *   of SM-count 32 KiB segments, one segment per CTA, every segment set up from scratch,
  *   each group with its own bucket scatter; no graph. */
@@ -102,10 +103,10 @@ typedef mp_range_stats mp_block_stats;
 
 typedef struct {
     uint32_t mode;          /* MP_MODE_BATCHED (default) or MP_MODE_PLAIN */
-    uint32_t tile_log2;     /* bits per tile: 0 = autotuned, else 18, 19 or 20 */
+    uint32_t tile_log2;     /* bits per odd-only tile: 0 = the handle's form, else 18..20 */
     uint32_t block_log2;    /* per-block stats width (integers); 0 = none; else >= tile_log2+1 */
     uint32_t hash_log2;     /* hash segment width (integers); 0 = no hashes; else 4..40 */
-    uint32_t threads;       /* threads per CTA: 0 = autotuned, else 256, 512 or 1024 */
+    uint32_t threads;       /* threads per CTA of odd-only tiles: 0 = the handle's form, else 256, 512, 1024 */
     uint32_t reserved[3];
 } mp_sieve_opts;
 
@@ -289,16 +290,15 @@ int mp_wieferich_stats_noalloc(const uint64_t *d_p, const uint64_t *d_q, uint64_
                                mp_wief_stats *d_stats, void *stream);
 
 /* ---- autotuner ----
- * Times the sieve tile geometry (tile bits x threads) on a short range at height `lo`
- * and the Fermat kernel variants, and keeps the fastest per handle.  Called implicitly
- * (on a small range) by the first call that needs it; call it explicitly to tune for a
- * given height.  *report receives a short text summary (nullable, cap bytes). */
+ * Times the sieve's residue planes and its odd-only tile geometries (tile bits x threads) on
+ * 2^34 integers at height `lo`, the Fermat kernel variants and the base-2 launch's CTA sizes,
+ * and keeps the fastest per handle.  *report receives a short text summary (nullable, cap bytes). */
 int mp_autotune(mp_handle *h, uint64_t lo, char *report, size_t cap);
 
 /* Sets one of the autotuner's choices on the handle, as mp_autotune would (so that callers
  * and tests can pin each one):
- *   MP_TUNE_TILE_LOG2      sieve tile bits (0 = default, 18, 19, 20)
- *   MP_TUNE_THREADS        sieve threads per CTA (0 = default, 256, 512, 1024)
+ *   MP_TUNE_TILE_LOG2      bits of an odd-only sieve tile (18, 19, 20), 0: not pinned
+ *   MP_TUNE_THREADS        threads per CTA of those tiles (256, 512, 1024), 0: not pinned
  *   MP_TUNE_SCATTER_STAGED 1: the staged bucket scatter, 0: the binned one
  *   MP_TUNE_BUCKET_DIV     primes above tile bits / value (1, 2 or 4) go to the buckets
  *   MP_TUNE_NO_PIPELINE    1: batched sieve calls as a host loop of wave launches, 0: one
@@ -306,6 +306,8 @@ int mp_autotune(mp_handle *h, uint64_t lo, char *report, size_t cap);
  *                          staged scatter always runs the wave loop)
  *   MP_TUNE_BPSW_VARIANT   0..3: threads per CTA of the batched base-2 launch
  *   MP_TUNE_FERMAT_ILP2    1: two primes per thread in the Fermat kernel
+ * Batched sieve calls run in residue planes mod 30, which size themselves, unless one of the
+ * first four is set to other than its default (0, 0, 1, 1).
  * Returns MP_EINVAL for an unknown knob or a value out of range.  No reference counterpart
  * (the reference picks its wheel and chunk by a cost model, A350826/a350826.c:1976-2015). */
 #define MP_TUNE_TILE_LOG2 1

@@ -121,7 +121,9 @@ __device__ __forceinline__ void plane_presieve(u32 *sm, u32 nw, const PlaneTileA
 }
 
 // CTA b sieves the tiles [b per, (b + 1) per) of the wave in order; tile t is block t mod nb of
-// plane t / nb, so that the thread-tier primes carry their next multiple along a plane
+// plane t / nb, so that the thread-tier primes carry their next multiple along a plane.  Bound by
+// shared-memory atomics: [1e15, +2^34) 3.45 ms, 1.75e12 marks and records a second or 0.88 of the rate of
+// atomics on random words (the odd-only tiles: 5.85 ms with their scans of 1.2, 0.51 of that rate)
 template <int NTH>
 __global__ void __launch_bounds__(NTH) plane_tile_kernel(PlaneTileArgs a)
 {
@@ -392,7 +394,10 @@ __device__ __forceinline__ void plane_flush(const PlaneScatterArgs &a, u32 nt, u
 // of its multiples.  A thread holds one prime and the next hit of each plane, and files one hit per
 // plane and round; in plane order the eight starts follow from one remainder i0 mod q.  Warps take
 // runs of primes from a queue and hand them to the lanes that have none, so no lane waits for a
-// neighbour with more hits; the queue replaces bounds computed on the host for each range.  SMALL, for
+// neighbour with more hits; the queue replaces bounds computed on the host for each range.  Bound by the
+// stage's shared memory traffic and issue: 3.2e11 records a second at 1e15 (2.24 ms for 2^34 integers; the
+// odd-only wheel of 210, with 1/7 fewer records by half as many turns, 4.19 ms), 1.7e11 at 9e17, where a
+// prime has 7.5 hits for its set-up (2.2 ms for 2^32, 5.5 before).  SMALL, for
 // waves with few units of work or few hits (2^16 integers at 9e17: 754 -> 260 us of scatter; 2^28 at
 // 1e12: 88 -> 42 us): units cover parts of the wave, a round looks for primes with hits up to eight
 // times, and primes far apart are first asked for any multiple at all.
@@ -700,6 +705,8 @@ __device__ __forceinline__ u32 run_starts(u32 any, u32 next, bool prev, u32 Z)
 // ANDs of planes.  The widest gap is found from the empty blocks: a run of z of them lies in a gap
 // between 30 z + 2 and 30 z + 58, so once a gap of g is known only runs of at least (g - 28) / 30
 // empty blocks are looked at, which are rare.  Until that is at least 1 the row's primes are walked.
+// 0.43 ms for 2^33 integers without the bitmap (4.6 GB of planes a ms: issue and the latency of a row),
+// 0.6 in the odd-only tiles; a short range waits some 20 us for one stretch's rows
 template <bool BITMAP>
 __global__ void __launch_bounds__(32 * SCAN_WARPS, 2) plane_scan_kernel(PlaneScanArgs a)
 {
