@@ -44,7 +44,7 @@ class Wief(C.Structure):
 
 def build(ref=True):
     """Compile liboracle.so, and the reference checkers when the reference tree exists."""
-    target = "ref" if ref and os.path.isdir(REFERENCE_TREE) else "all"
+    target = "ref" if ref and os.path.isdir(REFERENCE_TREE) and os.listdir(REFERENCE_TREE) else "all"
     subprocess.run(["make", "-s", "-C", HERE, target, f"MATHPUB_REFERENCE={REFERENCE_TREE}"], check=True)
 
 
