@@ -704,7 +704,10 @@ __device__ __forceinline__ u32 run_starts(u32 any, u32 next, bool prev, u32 Z)
 // 32 blocks of 30 integers, eight words, one per plane.  Counts are popcounts; twins and 6-tuples are
 // ANDs of planes.  The widest gap is found from the empty blocks: a run of z of them lies in a gap
 // between 30 z + 2 and 30 z + 58, so once a gap of g is known only runs of at least (g - 28) / 30
-// empty blocks are looked at, which are rare.  Until that is at least 1 the row's primes are walked.
+// empty blocks can hold a wider one, and of at least (g - 30) / 30 one as wide, which are rare.  A gap as
+// wide counts where it may come first: against another warp's, and in the row whose own search for long
+// runs first gave g, since the earliest of equal gaps can have a block fewer than the one found.  Until (g - 30) / 30 is at
+// least 1 the row's primes are walked.
 // 0.43 ms for 2^33 integers without the bitmap (4.6 GB of planes a ms: issue and the latency of a row),
 // 0.6 in the odd-only tiles; a short range waits some 20 us for one stretch's rows
 template <bool BITMAP>
@@ -834,7 +837,8 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS, 2) plane_scan_kernel(PlaneSca
                 if (lane == 0) atomicMax(&s_best, r);
             }
         };
-        if (best < 58) {
+        const bool first = best < 60;                    // no threshold from the rows before
+        if (first) {
             // the longest runs of the row first, which settles the threshold at once at most heights
             for (u32 Z = 16; Z; Z >>= 1) {
                 const u32 st = run_starts(any, nxt, prev, Z);
@@ -846,7 +850,7 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS, 2) plane_scan_kernel(PlaneSca
                 }
             }
         }
-        const bool walk = best < 58;
+        const bool walk = best < 60;
         if (walk || walked) {
             // exact primes of the row's words: the lane's first and last, and the last before the lane
             u32 pm[8];
@@ -888,8 +892,10 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS, 2) plane_scan_kernel(PlaneSca
             walked = walk || !rl;
         }
         if (!walk) {
-            // a gap found by another warp counts too, but one that ties it may come first here
-            const u32 other = *(volatile u32 *)&s_best, Z = max(best - 28, other > 30 ? other - 30 : 0u) / 30;
+            // a gap found by another warp counts too, but one that ties it may come first here, as one that ties
+            // this row's own first find may
+            const u32 other = *(volatile u32 *)&s_best;
+            const u32 Z = max(best - (first ? 30 : 28), other > 30 ? other - 30 : 0u) / 30;
             const u32 st = run_starts(any, nxt, prev, min(32u, Z));
             if (__any_sync(0xffffffffu, st != 0)) {
                 close_runs(st);
