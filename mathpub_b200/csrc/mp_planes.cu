@@ -20,6 +20,7 @@
 // Reference behaviour (paths inside the Mathpub project): see mp_sieve.cu; the mod-30 layout is
 // the one of A158939/cuda/a158939_cuda.cu:26-41 with a plane instead of a bit per residue.
 #include "mp_sieve.cuh"
+#include "mp_planes_cap.h"
 #include <algorithm>
 #include <math.h>
 
@@ -1163,9 +1164,7 @@ static int plan_planes(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, P
         if (P.iend - P.it1 <= 16 * P.threads) P.it1 = P.iend;
         P.cap = 0;
         if (P.iend > P.it1) {
-            // expected records of a tile: each bucket prime hits a block of pt bits pt / q times
-            const double e = (double)P.pt * (tb.inv_prefix[P.iend] - tb.inv_prefix[P.it1]);
-            P.cap = ((u32)(e * 1.02 + 10.0 * sqrt(e + 1.0) + 256.0) + 3) & ~3u;
+            P.cap = plane_bucket_cap(P.pt, tb.inv_prefix[P.iend] - tb.inv_prefix[P.it1], g.base / 30, tb.host[P.iend - 1]);
             // records of a wave within 3 GB
             if ((u64)P.cap * 8 * P.nb * 4 > (3072ull << 20) && P.tw > 1) continue;
         }
