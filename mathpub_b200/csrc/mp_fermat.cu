@@ -344,9 +344,10 @@ __device__ __forceinline__ FermOut fermat_one(u64 p)
 
 // one prime per thread (ILP = 1) or two interleaved primes per thread (ILP = 2).  The entries that
 // are not ok are done again at the end, from the definition: inside the loop that code cost the
-// ladder registers (5% of the kernel), and no prime needs it
+// ladder registers (5% of the kernel), and no prime needs it.  Until then such an entry holds its p
+// with bit 63 set (p and every quotient are below 2^63), so that Q may be P's own array
 template <int K, int ILP>
-__global__ void __launch_bounds__(256) fermat_kernel(const u64 *__restrict__ P, u64 count, u64 *Q)
+__global__ void __launch_bounds__(256) fermat_kernel(const u64 *P, u64 count, u64 *Q)
 {
     const u64 stride = (u64)gridDim.x * blockDim.x * ILP, first = ((u64)blockIdx.x * blockDim.x + threadIdx.x) * ILP;
     bool again = false;
@@ -355,20 +356,20 @@ __global__ void __launch_bounds__(256) fermat_kernel(const u64 *__restrict__ P, 
         FermOut o[ILP];
 #pragma unroll
         for (int v = 0; v < ILP; v++) {
-            p[v] = i + v < count ? __ldg(P + i + v) : 0;
+            p[v] = i + v < count ? P[i + v] : 0;
             o[v] = fermat_one<K>(p[v] >= 3 && (p[v] & 1) ? p[v] : 3);
         }
 #pragma unroll
         for (int v = 0; v < ILP; v++) {
             const bool odd = p[v] >= 3 && (p[v] & 1);
-            if (i + v < count) Q[i + v] = odd ? (o[v].ok ? o[v].q : ~0ull) : 0;
+            if (i + v < count) Q[i + v] = odd ? (o[v].ok ? o[v].q : p[v] | 1ull << 63) : 0;
             again |= odd && !o[v].ok;
         }
     }
     if (!again) return;
     for (u64 i = first; i < count; i += stride)
         for (int v = 0; v < ILP; v++)
-            if (i + v < count && Q[i + v] == ~0ull) Q[i + v] = fermat_not_one<K>(__ldg(P + i + v));
+            if (i + v < count && Q[i + v] >> 63) Q[i + v] = fermat_not_one<K>(Q[i + v] & ~(1ull << 63));
 }
 
 // ---- statistics: checksum, near count, FLT errors, hits, ordered hash ----
