@@ -1017,9 +1017,12 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS, 2) plane_scan_kernel(PlaneSca
 // the in-range primes of each stretch, in order, from place emit_off on.  A warp takes 32 words (1024
 // blocks of 30) at a time: the lanes put their primes as 16-bit offsets into the warp's part of shared
 // memory, and the warp writes them out in whole rows (36 M primes near 1e12: 0.13 ms, 0.44 with every
-// lane writing its own run)
+// lane writing its own run).  Its part holds as many as any window of 30720 integers is known to have
+// (pi(30720) = 3314); that no window has more is not proved, so a row of more is written lane by lane
 #define EMIT_WARPS 8
-#define EMIT_ROW 3328u                 // 30720 consecutive integers hold at most pi(30720) = 3313 primes above 5
+#ifndef EMIT_ROW
+#define EMIT_ROW 3328u
+#endif
 __global__ void __launch_bounds__(32 * EMIT_WARPS) plane_emit_kernel(PlaneScanArgs a)
 {
     extern __shared__ __align__(16) u16 s_offs[];         // [EMIT_WARPS][EMIT_ROW]
@@ -1062,19 +1065,22 @@ __global__ void __launch_bounds__(32 * EMIT_WARPS) plane_emit_kernel(PlaneScanAr
         }
         u32 v[8], pos = incl - c;
         transpose_planes(v, p);
+        const u64 first = 30 * (a.i0 + (u64)(wr + 32 * warp) * 32), to = at + before;
+        const bool staged = n <= EMIT_ROW;                // the same in the whole warp
 #pragma unroll
         for (int m = 0; m < 8; m++) {
             const u32 x0 = 30 * (32 * lane + 4 * m);
             for (u32 y = v[m]; y; y &= y - 1) {           // four blocks, a byte each
-                const u32 k = __ffs(y) - 1;
-                if (pos < EMIT_ROW) out[pos] = (u16)(x0 + 30 * (k >> 3) + (__byte_perm(0x0d0b0701u, 0x1d171311u, k & 7) & 0xffu));
+                const u32 k = __ffs(y) - 1, x = x0 + 30 * (k >> 3) + (__byte_perm(0x0d0b0701u, 0x1d171311u, k & 7) & 0xffu);
+                if (staged) out[pos] = (u16)x;
+                else if (to + pos < a.emit_cap) a.emit[to + pos] = first + x;
                 pos++;
             }
         }
         __syncwarp();
-        const u64 x0 = 30 * (a.i0 + (u64)(wr + 32 * warp) * 32), to = at + before;
-        for (u32 i = lane; i < n; i += 32)
-            if (to + i < a.emit_cap) __stcs(a.emit + to + i, x0 + out[i]);
+        if (staged)
+            for (u32 i = lane; i < n; i += 32)
+                if (to + i < a.emit_cap) __stcs(a.emit + to + i, first + out[i]);
         at += total;
         __syncthreads();
     }
