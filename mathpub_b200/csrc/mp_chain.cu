@@ -761,8 +761,25 @@ void mp_chain_free(mp_handle *h)
 #define CS_WIDE_MIN (6ull << 44)
 #define CS_DEEP_MIN (1ull << 39)
 
+static int cs_upload(mp_handle *h, ChainDev &D)
+{
+    const CsPlan &P = D.plan;
+    if (D.ok) {
+        MP_CUDA(h, upload(D.ginfo, P.ginfo));
+        MP_CUDA(h, upload(D.q, P.q));
+        MP_CUDA(h, upload(D.qinv, P.qinv));
+        MP_CUDA(h, upload(D.crt, P.crt));
+        MP_CUDA(h, upload(D.pat, P.pat));
+        MP_CUDA(h, upload(D.res, P.res));
+    }
+    MP_CUDA(h, upload(D.offs, P.offs));
+    MP_CUDA(h, D.cnt.ensure((CS_NCNT + 3) * sizeof(ull)));
+    return MP_OK;
+}
+
 // the handle's plan for (mode, offs) and a range of `len` integers, built and uploaded when it is none
-// of the last two
+// of the last two.  The handle gets a plan only when all its tables are on the device; without room for
+// two, the former plan goes
 static int cs_prepare(mp_handle *h, u32 mode, const std::vector<u32> &offs, u128t len)
 {
     const u32 tier = len >= CS_WIDE_MIN ? 2 : len >= CS_DEEP_MIN ? 1 : 0;
@@ -780,25 +797,25 @@ static int cs_prepare(mp_handle *h, u32 mode, const std::vector<u32> &offs, u128
         delete keep->other;
         keep->other = nullptr;
     }
-    h->chain = new ChainDev();
-    h->chain->other = keep;
-    h->chain->tier = tier;
-    ChainDev &D = *h->chain;
-    D.mode = mode;
-    D.k = (u32)offs.size();
-    D.key = offs;
-    D.ok = make_plan(offs, tier, D.plan);
-    const CsPlan &P = D.plan;
-    if (D.ok) {
-        MP_CUDA(h, upload(D.ginfo, P.ginfo));
-        MP_CUDA(h, upload(D.q, P.q));
-        MP_CUDA(h, upload(D.qinv, P.qinv));
-        MP_CUDA(h, upload(D.crt, P.crt));
-        MP_CUDA(h, upload(D.pat, P.pat));
-        MP_CUDA(h, upload(D.res, P.res));
+    ChainDev *const D = new ChainDev();
+    D->tier = tier;
+    D->mode = mode;
+    D->k = (u32)offs.size();
+    D->key = offs;
+    D->ok = make_plan(offs, tier, D->plan);
+    int rc = cs_upload(h, *D);
+    if (rc == MP_ENOMEM && keep) {
+        mp_chain_free(h);
+        keep = nullptr;
+        rc = cs_upload(h, *D);
     }
-    MP_CUDA(h, upload(D.offs, P.offs));
-    MP_CUDA(h, D.cnt.ensure((CS_NCNT + 3) * sizeof(ull)));
+    if (rc != MP_OK) {
+        D->release();
+        delete D;
+        return rc;
+    }
+    D->other = keep;
+    h->chain = D;
     return MP_OK;
 }
 

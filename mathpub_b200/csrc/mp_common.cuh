@@ -133,6 +133,10 @@ struct DevBuf {
         size_t b = (need < 256 ? 256 : need) + spare;
         cudaError_t e = cudaMalloc(&p, b);
         if (e == cudaSuccess) bytes = b;
+        else {
+            p = nullptr;
+            cudaGetLastError();                            // reported by the caller, not by a later launch
+        }
         return e;
     }
     void release()

@@ -1,0 +1,65 @@
+"""Calls on a device with little free memory: one that cannot have its tables fails with MP_ENOMEM and leaves the
+handle as it was, so that the same call succeeds once there is memory."""
+import numpy as np
+import pytest
+
+import mathpub_b200 as mp
+
+pytestmark = pytest.mark.gpu
+
+SEXT = (0, 4, 6, 10, 12, 16)
+
+
+class Ballast:
+    """Holds the device's free memory but for `leave` bytes."""
+
+    def __init__(self, leave):
+        self.leave, self.held = leave, []
+
+    def __enter__(self):
+        import torch
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        size = 1 << 36
+        while size >= 1 << 21:
+            free = torch.cuda.mem_get_info()[0] - self.leave
+            if free >= size + (1 << 22):
+                try:
+                    self.held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+                    continue
+                except torch.OutOfMemoryError:
+                    pass
+            size >>= 1
+        return self
+
+    def __exit__(self, *a):
+        import torch
+        self.held.clear()
+        torch.cuda.empty_cache()
+
+
+def enomem(call):
+    with pytest.raises(mp.MathpubError) as x:
+        call()
+    assert x.value.code == mp.MP_ENOMEM
+
+
+def test_constellation_tables():
+    lo, n = 10 ** 15, 10 ** 12
+    with mp.Engine(0) as other:
+        want = other.tuple_count(lo, lo + n, SEXT), other.chain_sieve(lo, lo + n, 10)
+    with mp.Engine(0) as e:
+        e.sieve_range(10 ** 9, 10 ** 9 + 1000)
+        with Ballast(4 << 20):
+            enomem(lambda: e.tuple_count(lo, lo + n, SEXT))
+            enomem(lambda: e.tuple_count(lo, lo + n, SEXT))
+        assert e.tuple_count(lo, lo + n, SEXT) == want[0]
+        with Ballast(4 << 20):                               # a plan on the handle, no room for another beside it
+            try:
+                h, l = e.chain_sieve(lo, lo + n, 10)
+                assert np.array_equal(h, want[1][0]) and np.array_equal(l, want[1][1])
+            except mp.MathpubError as x:
+                assert x.code == mp.MP_ENOMEM
+        h, l = e.chain_sieve(lo, lo + n, 10)
+        assert np.array_equal(h, want[1][0]) and np.array_equal(l, want[1][1])
+        assert e.tuple_count(lo, lo + n, SEXT) == want[0]
