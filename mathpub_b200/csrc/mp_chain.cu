@@ -731,6 +731,15 @@ struct ChainDev {
     std::vector<u128t> kept_h;
     std::vector<u32> kept_l;
     DevBuf ginfo, q, qinv, crt, pat, res, offs, bq, l0, l1, cnt, rh, rl;
+    // the work lists, which no call leaves anything in: they go from plan to plan
+    void take_lists(ChainDev &from)
+    {
+        std::swap(bq, from.bq);
+        std::swap(l0, from.l0);
+        std::swap(l1, from.l1);
+        std::swap(rh, from.rh);
+        std::swap(rl, from.rl);
+    }
     void release()
     {
         for (DevBuf *b : {&ginfo, &q, &qinv, &crt, &pat, &res, &offs, &bq, &l0, &l1, &cnt, &rh, &rl}) b->release();
@@ -790,6 +799,7 @@ static int cs_prepare(mp_handle *h, u32 mode, const std::vector<u32> &offs, u128
         h->chain = keep->other;
         keep->other = nullptr;
         h->chain->other = keep;
+        h->chain->take_lists(*keep);
         return MP_OK;
     }
     if (keep && keep->other) {
@@ -815,6 +825,7 @@ static int cs_prepare(mp_handle *h, u32 mode, const std::vector<u32> &offs, u128
         return rc;
     }
     D->other = keep;
+    if (keep) D->take_lists(*keep);
     h->chain = D;
     return MP_OK;
 }

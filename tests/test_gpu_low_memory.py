@@ -63,3 +63,27 @@ def test_constellation_tables():
         h, l = e.chain_sieve(lo, lo + n, 10)
         assert np.array_equal(h, want[1][0]) and np.array_equal(l, want[1][1])
         assert e.tuple_count(lo, lo + n, SEXT) == want[0]
+
+
+def test_two_plans_share_the_work_lists():
+    """Two patterns used in turn on one handle hold the work lists once (about 0.5 GB here), not once each."""
+    import torch
+    lo, n = 10 ** 15, 2 * 10 ** 11
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    with mp.Engine(0) as other:
+        want = other.tuple_count(lo, lo + n, (0, 2, 6, 8)), other.tuple_count(lo, lo + n, (0, 4, 6, 10))
+    with mp.Engine(0) as e:
+        before = free()
+        assert e.tuple_count(lo, lo + n, (0, 2, 6, 8)) == want[0]
+        one = free()
+        assert e.tuple_count(lo, lo + n, (0, 4, 6, 10)) == want[1]
+        two = free()
+        assert before - one > 200 << 20 and one - two < 100 << 20
+        for _ in range(2):
+            assert e.tuple_count(lo, lo + n, (0, 2, 6, 8)) == want[0]
+            assert e.tuple_count(lo, lo + n, (0, 4, 6, 10)) == want[1]
+        assert two - free() < 32 << 20
