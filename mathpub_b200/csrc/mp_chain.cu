@@ -783,6 +783,7 @@ void mp_chain_free(mp_handle *h)
 // 0.72 ms, so not below; to 2039 2.9 ms; 9 to 11 members to 1021: 302 -> 423 ms).
 #define CS_WIDE_MIN (6ull << 44)
 #define CS_DEEP_MIN (1ull << 39)
+static u32 cs_tier(u128t len) { return len >= CS_WIDE_MIN ? 2 : len >= CS_DEEP_MIN ? 1 : 0; }
 
 static int cs_upload(mp_handle *h, ChainDev &D)
 {
@@ -800,12 +801,11 @@ static int cs_upload(mp_handle *h, ChainDev &D)
     return MP_OK;
 }
 
-// the handle's plan for (mode, offs) and a range of `len` integers, built and uploaded when it is none
+// the handle's plan for (mode, offs) and the tier, built and uploaded when it is none
 // of the last two.  The handle gets a plan only when all its tables are on the device; without room for
 // two, the former plan goes
-static int cs_prepare(mp_handle *h, u32 mode, const std::vector<u32> &offs, u128t len)
+static int cs_prepare(mp_handle *h, u32 mode, const std::vector<u32> &offs, u32 tier)
 {
-    const u32 tier = len >= CS_WIDE_MIN ? 2 : len >= CS_DEEP_MIN ? 1 : 0;
     const auto fits = [&](const ChainDev *c) { return c && c->mode == mode && c->tier == tier && c->key == offs; };
     if (fits(h->chain)) return MP_OK;
     ChainDev *keep = h->chain;                             // it becomes the other one
@@ -964,7 +964,7 @@ static const u128t CS_HI128_MAX = (u128t)MP_CHAIN128_HI_MAX_W1 << 64 | MP_CHAIN1
 static int cs_chains(mp_handle *h, u128t lo, u128t hi, u32 k, u32 shape, std::vector<u128t> &H, std::vector<u32> &L)
 {
     cudaStream_t st = h->stream;
-    MP_TRY(cs_prepare(h, shape, chain_offsets(k, shape), hi - lo));
+    MP_TRY(cs_prepare(h, shape, chain_offsets(k, shape), cs_tier(hi - lo)));
     ChainDev &D = *h->chain;
     if (D.kept && D.kept_lo == lo && D.kept_hi == hi) {
         H.swap(D.kept_h);
@@ -1042,21 +1042,30 @@ extern "C" int mp_chain_sieve128(mp_handle *h, const uint64_t lo[2], const uint6
 
 // the first chain: runs in ascending order, stopping after the first run that holds one; the
 // smallest key wins (the head for gaps 2, 4, ...; for ..., 4, 2 the start of the k-prime
-// pattern that ends the chain, member len - k of it)
+// pattern that ends the chain, member len - k of it).  A short pattern has its first chain near lo however
+// long the range is, and a run takes a whole segment, which the larger wheel makes 23 times as long: so the
+// range's first CS_WIDE_MIN integers go with the plan of the shortest ranges (from 1e16 to 2^63 at k = 4: 12 ms,
+// 285 with the long range's plan; k = 8 2.5 and 8.8), and only the rest with the plan for its length (k = 14 over
+// 1e16 integers without one: 1.2 s)
 static int cs_first(mp_handle *h, u128t lo, u128t hi, u32 k, u32 shape, u128t *key, u128t *head, u32 *len)
 {
     cudaStream_t st = h->stream;
-    MP_TRY(cs_prepare(h, shape, chain_offsets(k, shape), hi - lo));
-    ChainDev &D = *h->chain;
-    D.kept = false;
     std::vector<u128t> H;
     std::vector<u32> L;
-    MP_TRY(cs_sieve_range(
-        h, D, lo, hi, st,
-        [&](const u64 *list, const ull *nin, u64 cap_, u128t base, u64 expect) {
-            return cs_collect(h, D, list, nin, cap_, base, expect, H, L, st);
-        },
-        [&]() { return !H.empty(); }));
+    for (u128t a = lo; a < hi && H.empty();) {
+        const bool near = a == lo;
+        const u128t b = near && hi - lo > CS_WIDE_MIN ? lo + CS_WIDE_MIN : hi;
+        MP_TRY(cs_prepare(h, shape, chain_offsets(k, shape), near ? 0 : cs_tier(b - a)));
+        ChainDev &D = *h->chain;
+        D.kept = false;
+        MP_TRY(cs_sieve_range(
+            h, D, a, b, st,
+            [&](const u64 *list, const ull *nin, u64 cap_, u128t base, u64 expect) {
+                return cs_collect(h, D, list, nin, cap_, base, expect, H, L, st);
+            },
+            [&]() { return !H.empty(); }));
+        a = b;
+    }
     for (size_t i = 0; i < H.size(); i++) {
         const u64 j = L[i] - k;
         const u128t kk = shape == 0 ? H[i] : H[i] + (u128t)(j * (2 * (u64)L[i] - 1 - j));
@@ -1118,7 +1127,7 @@ static int cs_tuples(mp_handle *h, u128t lo, u128t hi, const uint32_t *offs, uin
                      uint64_t *cks)
 {
     cudaStream_t st = h->stream;
-    MP_TRY(cs_prepare(h, CS_MODE_TUPLE, std::vector<u32>(offs, offs + k), hi - lo));
+    MP_TRY(cs_prepare(h, CS_MODE_TUPLE, std::vector<u32>(offs, offs + k), cs_tier(hi - lo)));
     ChainDev &D = *h->chain;
     ull *acc = D.cnt.as<ull>() + CS_CNT_TUPLE;
     MP_CUDA(h, cudaMemsetAsync(acc, 0, 2 * sizeof(ull), st));
