@@ -215,6 +215,8 @@ struct mp_handle {
     // scratch
     DevBuf tilesum, blockacc, rec, reccnt, queue, errflag, scratch_bitmap, bpsw_n, bpsw_bits, bpsw_list,
         ferm_p, ferm_q, ferm_part, stats_out, small_out, tstate, gap_acc, planes, emit_off;
+    u64 planes_max = ~0ull;          // bytes of a wave's buffers in the residue planes, once the device had no room for
+                                     // more; kept, so that a call and its capture take the same waves
     // CTA bounds of the bucket scatter, one buffer per (first prime, end prime, CTAs): a
     // captured graph reads the buffer it was captured with, so a buffer's contents are never
     // rewritten; the least recently used one is freed (which invalidates the graphs) when a

@@ -1134,7 +1134,29 @@ struct PlanePlan {
     u32 iw0, iw1, it1, iend;
     u32 cap;
     u64 ni;                           // plane bits of a full wave
+    u32 grid, nmod;                   // CTAs of the tile launch; primes of the remainders' launch
+    size_t psize, tsize, rsize;       // bytes of the planes, the threads' state and the records
 };
+
+static void (*const kTile[3])(PlaneTileArgs) = {plane_tile_kernel<256>, plane_tile_kernel<512>, plane_tile_kernel<1024>};
+static int tile_form(u32 threads) { return threads == 1024 ? 2 : threads == 512 ? 1 : 0; }
+
+// the buffers' bytes of a plan, without what they may have to spare
+static int plan_sizes(mp_handle *h, PlanePlan &P)
+{
+    static bool done[3][16] = {{false}};
+    const int tk = tile_form(P.threads);
+    MP_CUDA(h, raise_smem(kTile[tk], done[tk], h->device, (int)(PL_PTMAX / 8)));
+    int occ = 0;
+    MP_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kTile[tk], (int)P.threads, P.pt / 8));
+    const u32 ntile = 8 * P.nb;
+    P.grid = (u32)std::min<u64>(ntile, (u64)h->sm_count * (u32)std::max(occ, 1));
+    P.nmod = P.it1 - P.iw0 >= PL_IMOD_MIN ? P.it1 - P.iw0 : 0;
+    P.psize = ((size_t)ntile * (P.pt / 32) + 64) * 4;
+    P.tsize = ((size_t)P.grid * (P.it1 - P.iw1) + P.nmod) * 4 + 64;
+    P.rsize = P.cap ? (size_t)ntile * P.cap * 4 : 0;
+    return MP_OK;
+}
 
 static int plan_planes(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, PlanePlan &P)
 {
@@ -1174,6 +1196,8 @@ static int plan_planes(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, P
             // records of a wave within 3 GB
             if ((u64)P.cap * 8 * P.nb * 4 > (3072ull << 20) && P.tw > 1) continue;
         }
+        MP_TRY(plan_sizes(h, P));
+        if (P.psize + P.tsize + P.rsize > h->planes_max && P.tw > 1) continue;
         return MP_OK;
     }
 }
@@ -1190,34 +1214,34 @@ int mp_planes_shape(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, u32 
 int mp_planes_run(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, TileSum *sums, u32 *bitmap32, u64 *emit,
                   u64 emit_cap, u64 *emit_total, cudaStream_t st)
 {
-    static bool tile_done[3][16] = {{false}}, scat_done[2][16] = {{false}};
+    static bool scat_done[2][16] = {{false}};
     PlanePlan P;
-    MP_TRY(plan_planes(h, tb, g, P));
     int smem_max = 0;
     MP_CUDA(h, cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
-    const int tk = P.threads == 1024 ? 2 : P.threads == 512 ? 1 : 0;
-    static void (*const tile[3])(PlaneTileArgs) = {plane_tile_kernel<256>, plane_tile_kernel<512>, plane_tile_kernel<1024>};
-    MP_CUDA(h, raise_smem(tile[tk], tile_done[tk], h->device, (int)(PL_PTMAX / 8)));
-    const u32 ntile = 8 * P.nb, nw = P.pt / 32;
-    const size_t tsm = P.pt / 8;
-    int occ = 0;
-    MP_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, tile[tk], (int)P.threads, tsm));
-    const u32 grid = (u32)std::min<u64>(ntile, (u64)h->sm_count * (u32)std::max(occ, 1));
     // The buffers follow the range's length and, a little, its height; a growth frees the old one, which
     // waits for the device ([1e12 + x, +2^30) for growing x: 1.1 ms instead of 0.27).  So they grow with
     // something to spare; a third for the threads' state, which is largest below the longest waves
-    // (tiles of less than half an SM's shared memory run two to an SM).
-    const size_t spare = 32u << 20, psize = ((size_t)ntile * nw + 64) * 4;
-    MP_CUDA(h, h->planes.ensure(psize, psize / 16 + spare));
-    const u32 nmod = P.it1 - P.iw0 >= PL_IMOD_MIN ? P.it1 - P.iw0 : 0;
-    const size_t tsize = ((size_t)grid * (P.it1 - P.iw1) + nmod) * 4 + 64;
-    MP_CUDA(h, h->tstate.ensure(tsize, tsize / 3 + spare / 4));
-    const bool large = P.iend > P.it1;
-    if (large) {
-        const size_t rsize = (size_t)ntile * P.cap * 4;
-        MP_CUDA(h, h->rec.ensure(rsize, rsize / 16 + spare));
-        MP_CUDA(h, h->reccnt.ensure(((size_t)ntile + 1) * 4, 16384));
+    // (tiles of less than half an SM's shared memory run two to an SM).  Where the device has no room, they do
+    // without, and then with shorter waves (2^32 integers at 9e17 take 1.9 GB in one wave)
+    for (bool lean = false;;) {
+        MP_TRY(plan_planes(h, tb, g, P));
+        const size_t spare = lean ? 0 : 32u << 20;
+        cudaError_t e = h->planes.ensure(P.psize, lean ? 0 : P.psize / 16 + spare);
+        if (e == cudaSuccess) e = h->tstate.ensure(P.tsize, lean ? 0 : P.tsize / 3 + spare / 4);
+        if (e == cudaSuccess && P.cap) e = h->rec.ensure(P.rsize, lean ? 0 : P.rsize / 16 + spare);
+        if (e == cudaSuccess && P.cap) e = h->reccnt.ensure(((size_t)8 * P.nb + 1) * 4, 16384);
+        if (e == cudaSuccess) break;
+        if (e != cudaErrorMemoryAllocation || (lean && P.tw == 1)) MP_CUDA(h, e);
+        if (lean) h->planes_max = (P.psize + P.tsize + P.rsize) / 2;
+        lean = true;
+        h->planes.release();
+        h->tstate.release();
+        h->rec.release();
     }
+    const int tk = tile_form(P.threads);
+    const u32 ntile = 8 * P.nb, nw = P.pt / 32, grid = P.grid, nmod = P.nmod;
+    const size_t tsm = P.pt / 8;
+    const bool large = P.iend > P.it1;
     PlaneTileArgs a;
     memset(&a, 0, sizeof a);
     a.nb = P.nb; a.pt = P.pt; a.ntile = ntile;
@@ -1305,7 +1329,7 @@ int mp_planes_run(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, TileSu
         }
         {
             ProfScope ps(h, PROF_TILE, st);
-            tile[tk]<<<grid, P.threads, tsm, st>>>(a);
+            kTile[tk]<<<grid, P.threads, tsm, st>>>(a);
         }
         MP_CUDA(h, cudaGetLastError());
         c.t0 = t0;

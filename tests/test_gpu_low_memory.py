@@ -87,3 +87,30 @@ def test_two_plans_share_the_work_lists():
             assert e.tuple_count(lo, lo + n, (0, 2, 6, 8)) == want[0]
             assert e.tuple_count(lo, lo + n, (0, 4, 6, 10)) == want[1]
         assert two - free() < 32 << 20
+
+
+def stats(r):
+    return {k: r[k] for k in ("pi", "twins", "max_gap", "gap_start", "tuple6", "tuple6_cks", "first_prime", "last_prime")}
+
+
+def range_with(lo, n, leave):
+    """A range on a new handle, with `leave` bytes of device memory beside its tables."""
+    with mp.Engine(0) as other:
+        want = other.sieve_range(lo, lo + n)
+    with mp.Engine(0) as e:
+        e.sieve_range(lo + n - 2 ** 16, lo + n)
+        with Ballast(leave):
+            got = [e.sieve_range(lo, lo + n) for _ in range(4)]         # the later ones captured and replayed
+        assert all(stats(r) == stats(want) for r in got)
+        assert stats(e.sieve_range(lo, lo + n)) == stats(want)
+
+
+def test_range_without_room_to_spare():
+    """A wave's buffers take about 80 MB here, and half as much again with what they grow by beyond the need."""
+    range_with(10 ** 12, 2 ** 30, 60 << 20)
+
+
+@pytest.mark.parametrize("leave_mb", [1000, 400])
+def test_range_in_shorter_waves(leave_mb):
+    """One wave's buffers take 1.9 GB here."""
+    range_with(9 * 10 ** 17, 2 ** 32, leave_mb << 20)
