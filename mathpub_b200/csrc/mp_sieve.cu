@@ -2242,7 +2242,7 @@ int mp_sieve_emit_primes(mp_handle *h, u64 lo, u64 hi, u64 *d_primes, u64 cap, u
 // the primes of [lo, hi) into `buf`, grown to hold them; synchronises.  One pass over the range: the
 // buffer is sized by a bound on their number that fails only for ranges too short to matter (then a
 // second pass runs with the exact size): pi(x) < 1.2551 x / ln x, and for a range far from 0 its length
-// over ln lo with a margin
+// over ln lo with a margin.  Without room for that on the device, the primes are counted first
 int mp_primes_to_device(mp_handle *h, u64 lo, u64 hi, DevBuf &buf, u64 *count, cudaStream_t st)
 {
     *count = 0;
@@ -2251,8 +2251,14 @@ int mp_primes_to_device(mp_handle *h, u64 lo, u64 hi, DevBuf &buf, u64 *count, c
     double n = lo < hi / 16 ? 1.2551 * (double)hi / log((double)std::max<u64>(hi, 16)) : 1.06 * len / log((double)lo);
     n = std::min(n + 4.0 * sqrt(len) + 64.0, len);
     for (int pass = 0; pass < 2; pass++) {
-        const u64 cap = pass ? *count : (u64)n + 1;
-        MP_CUDA(h, buf.ensure((size_t)cap * 8 + 8));
+        u64 cap = pass ? *count : (u64)n + 1;
+        cudaError_t e = buf.ensure((size_t)cap * 8 + 8);
+        if (e == cudaErrorMemoryAllocation && !pass) {
+            MP_TRY(mp_sieve_emit_primes(h, lo, hi, nullptr, 0, count, st));
+            cap = *count;
+            e = buf.ensure((size_t)cap * 8 + 8);
+        }
+        MP_CUDA(h, e);
         MP_TRY(mp_sieve_emit_primes(h, lo, hi, buf.as<u64>(), cap, count, st));
         if (*count <= cap) return MP_OK;
     }

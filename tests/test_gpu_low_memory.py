@@ -114,3 +114,15 @@ def test_range_without_room_to_spare():
 def test_range_in_shorter_waves(leave_mb):
     """One wave's buffers take 1.9 GB here."""
     range_with(9 * 10 ** 17, 2 ** 32, leave_mb << 20)
+
+
+def test_prime_list_of_its_exact_size():
+    """The 1.63 GB of the primes below 2^32 fit, the 1.95 GB of the bound on their number do not."""
+    hi = 2 ** 32
+    with mp.Engine(0) as other:
+        want = other.wieferich_range(0, hi)
+    with mp.Engine(0) as e:
+        e.sieve_range(0, hi)                                          # the sieve's own buffers
+        with Ballast(1780 << 20):
+            got = e.wieferich_range(0, hi)
+    assert got == want
