@@ -1273,9 +1273,10 @@ __global__ void __launch_bounds__(32) hash_kernel(const u32 *__restrict__ bm, u6
     for (; k + 1 < nbytes && (((uintptr_t)(p + k)) & 15); k++) h.byte(p[k]);
     // whole blocks of HASH_AHEAD 16-byte words.  Each lane copies its block b + 1 to shared memory
     // (asynchronously) while block b is hashed from there: with plain loads the chains waited on them,
-    // 32 sectors a load (0.72 ms instead of 0.57)
+    // 32 sectors a load (0.72 ms instead of 0.57).  Segments of whole 16-byte words are all at the same distance k from
+    // a boundary (0, or 8 bytes where the caller's bitmap is)
     const u64 nblk = nbytes > k + 1 ? (nbytes - k - 1) / (16 * HASH_AHEAD) : 0;
-    const bool rows = (seg_bits & 127) == 0 && ((uintptr_t)bm & 15) == 0;        // then k = 0 everywhere
+    const bool rows = (seg_bits & 127) == 0;
     if (rows) {
         const u32 most = __reduce_max_sync(0xffffffffu, (u32)nblk);
         const u32 to = (u32)__cvta_generic_to_shared(&stage[0][lane * HASH_PITCH]);
@@ -1284,7 +1285,7 @@ __global__ void __launch_bounds__(32) hash_kernel(const u32 *__restrict__ bm, u6
 #pragma unroll
                 for (u32 i = 0; i < HASH_AHEAD; i++)
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::
-                                 "r"(to + (b & 1) * (32 * HASH_PITCH * 16) + 16 * i), "l"(p + 16 * (HASH_AHEAD * (u64)b + i))
+                                 "r"(to + (b & 1) * (32 * HASH_PITCH * 16) + 16 * i), "l"(p + k + 16 * (HASH_AHEAD * (u64)b + i))
                                  : "memory");
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
@@ -1454,8 +1455,8 @@ __global__ void __launch_bounds__(128) hash_rows_kernel(const u32 *__restrict__ 
 static void hash_launch(const u32 *bm, u64 nbits, u64 seg_bits, u64 nseg, u64 *out, cudaStream_t st)
 {
     // the parallel form for segments of a row and more, up to the count where it takes as long as the
-    // serial one (whose time does not depend on the count while each has a thread of its own)
-    if (seg_bits >= 8192 && nseg <= 11000) hash_rows_kernel<<<(unsigned)((nseg + 3) / 4), 128, 0, st>>>(bm, nbits, seg_bits, nseg, out);
+    // serial one (whose time does not depend on the count while each has a thread of its own).  It reads 64-bit words
+    if (seg_bits >= 8192 && nseg <= 11000 && ((uintptr_t)bm & 7) == 0) hash_rows_kernel<<<(unsigned)((nseg + 3) / 4), 128, 0, st>>>(bm, nbits, seg_bits, nseg, out);
     else hash_kernel<<<(unsigned)((nseg + 31) / 32), 32, 0, st>>>(bm, nbits, seg_bits, nseg, out);
 }
 
