@@ -317,6 +317,7 @@ int mp_sieve_emit_primes(mp_handle *h, u64 lo, u64 hi, u64 *d_primes, u64 cap, u
                          cudaStream_t st);                           // synchronises
 int mp_primes_to_device(mp_handle *h, u64 lo, u64 hi, DevBuf &buf, u64 *count, cudaStream_t st);
 int mp_sieve_errors(mp_handle *h, cudaStream_t st);                  // synchronises; reads the error flag
+extern "C" u64 mp_sieve_scratch(mp_handle *h, u64 lo, u64 hi);       // bytes that a range request holds while it runs
 int mp_bpsw_run(mp_handle *h, const u64 *d_n, const u64 *offs, const u32 *lens, u32 nlists,
                 u32 *d_bits, u32 mode, cudaStream_t st);             // mp_bpsw.cu
 const char *mp_bpsw_variant_name(int v);

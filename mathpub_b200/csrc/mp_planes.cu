@@ -22,6 +22,7 @@
 #include "mp_sieve.cuh"
 #include "mp_planes_cap.h"
 #include <algorithm>
+#include <atomic>
 #include <math.h>
 
 // c_res(k): the residues in order
@@ -1120,7 +1121,7 @@ __global__ void __launch_bounds__(1024) plane_offsets_kernel(const TileSum *sums
 
 // raise a kernel's limit on dynamic shared memory to the device's, once per device
 template <class F>
-static cudaError_t raise_smem(F kernel, bool (&done)[16], int device, int bytes)
+static cudaError_t raise_smem(F kernel, std::atomic<bool> (&done)[16], int device, int bytes)
 {
     if (device < 0 || device >= 16) return cudaErrorInvalidDevice;
     if (done[device]) return cudaSuccess;
@@ -1144,7 +1145,7 @@ static int tile_form(u32 threads) { return threads == 1024 ? 2 : threads == 512 
 // the buffers' bytes of a plan, without what they may have to spare
 static int plan_sizes(mp_handle *h, PlanePlan &P)
 {
-    static bool done[3][16] = {{false}};
+    static std::atomic<bool> done[3][16];
     const int tk = tile_form(P.threads);
     MP_CUDA(h, raise_smem(kTile[tk], done[tk], h->device, (int)(PL_PTMAX / 8)));
     int occ = 0;
@@ -1158,7 +1159,8 @@ static int plan_sizes(mp_handle *h, PlanePlan &P)
     return MP_OK;
 }
 
-static int plan_planes(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, PlanePlan &P)
+// most: the bytes that a wave's buffers may take (one stretch at the least)
+static int plan_planes(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, u64 most, PlanePlan &P)
 {
     const u64 S = 2ull << g.tlog, top = g.base + 2 * g.nbx;
     const u64 sq = mp_isqrt64(top - 1) + 1;
@@ -1197,7 +1199,7 @@ static int plan_planes(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, P
             if ((u64)P.cap * 8 * P.nb * 4 > (3072ull << 20) && P.tw > 1) continue;
         }
         MP_TRY(plan_sizes(h, P));
-        if (P.psize + P.tsize + P.rsize > h->planes_max && P.tw > 1) continue;
+        if (P.psize + P.tsize + P.rsize > most && P.tw > 1) continue;
         return MP_OK;
     }
 }
@@ -1205,16 +1207,24 @@ static int plan_planes(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, P
 int mp_planes_shape(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, u32 *tile_bits, u32 *bucket_above)
 {
     PlanePlan P;
-    MP_TRY(plan_planes(h, tb, g, P));
+    MP_TRY(plan_planes(h, tb, g, h->planes_max, P));
     *tile_bits = P.pt;
     *bucket_above = P.it1 ? tb.host[P.it1 - 1] : 0;
+    return MP_OK;
+}
+
+int mp_planes_bytes(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, u64 *bytes)
+{
+    PlanePlan P;
+    MP_TRY(plan_planes(h, tb, g, ~0ull, P));
+    *bytes = P.psize + P.tsize + P.rsize;
     return MP_OK;
 }
 
 int mp_planes_run(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, TileSum *sums, u32 *bitmap32, u64 *emit,
                   u64 emit_cap, u64 *emit_total, cudaStream_t st)
 {
-    static bool scat_done[2][16] = {{false}};
+    static std::atomic<bool> scat_done[2][16];
     PlanePlan P;
     int smem_max = 0;
     MP_CUDA(h, cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
@@ -1224,7 +1234,7 @@ int mp_planes_run(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, TileSu
     // (tiles of less than half an SM's shared memory run two to an SM).  Where the device has no room, they do
     // without, and then with shorter waves (2^32 integers at 9e17 take 1.9 GB in one wave)
     for (bool lean = false;;) {
-        MP_TRY(plan_planes(h, tb, g, P));
+        MP_TRY(plan_planes(h, tb, g, h->planes_max, P));
         const size_t spare = lean ? 0 : 32u << 20;
         cudaError_t e = h->planes.ensure(P.psize, lean ? 0 : P.psize / 16 + spare);
         if (e == cudaSuccess) e = h->tstate.ensure(P.tsize, lean ? 0 : P.tsize / 3 + spare / 4);
@@ -1344,7 +1354,7 @@ int mp_planes_run(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, TileSu
         if (emit_total) {
             plane_offsets_kernel<<<1, 1024, 0, st>>>(sums, t0, nt, off, emit_total);
             if (emit) {
-                static bool emit_done[16] = {false};
+                static std::atomic<bool> emit_done[16];
                 MP_CUDA(h, raise_smem(plane_emit_kernel, emit_done, h->device, EMIT_WARPS * EMIT_ROW * 2));
                 plane_emit_kernel<<<nt, 32 * EMIT_WARPS, EMIT_WARPS * EMIT_ROW * 2, st>>>(c);
             }

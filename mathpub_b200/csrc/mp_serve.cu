@@ -67,15 +67,7 @@ static double now_s()
     return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
 
-// device memory a request occupies while it runs (scratch of its launch)
-static u64 range_mem(u64 lo, u64 hi)
-{
-    const u64 bits = (hi + MP_TAIL - (lo & ~1ull)) / 2;
-    const u64 tiles = (bits >> 20) + 1;
-    const u64 wave = std::min<u64>(tiles, 1184);
-    return tiles * 64 + wave * (1ull << 20) + (1ull << 20);
-}
-
+// device memory a primality request occupies while it runs (a range request's: mp_sieve_scratch)
 static u64 bpsw_mem(u64 count) { return count * 8 + count / 8 + 4096; }
 
 // the next chunk of a range request, joined into its result; true when the range is done
@@ -308,7 +300,7 @@ int mp_serve_submit_range(mp_server *s, uint64_t lo, uint64_t hi, uint64_t *req_
     // integers each), so a turn covers at least 64 integers per sieving prime up to sqrt(hi)
     const u64 np = s->main->tab->count_le(mp_isqrt64(hi + MP_TAIL - 1));
     r->chunk = std::max<u64>(s->chunk, 64 * np);
-    r->mem = range_mem(lo, hi - lo > r->chunk ? lo + r->chunk : hi);   // one chunk in flight
+    r->mem = mp_sieve_scratch(s->main, hi - lo > r->chunk ? hi - r->chunk : lo, hi);   // one chunk in flight, the highest
     r->res.kind = 1;
     return submit(s, r, req_id);
 }

@@ -2096,6 +2096,25 @@ int mp_planes_geom(mp_handle *h, u64 lo, u64 hi, u32 block_log2, SieveGeom &g)
     return MP_OK;
 }
 
+// the device memory of a batched range without hashes or a bitmap, with the handle's prime table reaching
+// sqrt(hi): its wave's buffers (2^32 integers near 1e18: 1.9 GB, mostly records of the bucket primes) and 64
+// bytes a stretch; in the odd-only tiles 1 MB each of a wave's tiles
+extern "C" u64 mp_sieve_scratch(mp_handle *h, u64 lo, u64 hi)
+{
+    SieveGeom g;
+    u64 b = 0;
+    if (planes_form(h, nullptr) && mp_planes_geom(h, lo, hi, 0, g) == MP_OK) {
+        int dev = 0;
+        cudaGetDevice(&dev);                             // the caller's, put back
+        cudaSetDevice(h->device);
+        const int rc = mp_planes_bytes(h, *h->tab, g, &b);
+        cudaSetDevice(dev);
+        if (rc == MP_OK) return b + (u64)g.ntiles * sizeof(TileSum) + (1ull << 20);
+    }
+    const u64 tiles = ((hi + MP_TAIL - (lo & ~1ull)) / 2 >> 20) + 1;
+    return tiles * 64 + std::min<u64>(tiles, 1184) * (1ull << 20) + (1ull << 20);
+}
+
 int mp_sieve_run(mp_handle *h, u64 lo, u64 hi, const mp_sieve_opts *o, mp_range_stats *d_out,
                  mp_block_stats *d_blocks, u64 *d_hash, u64 *d_bitmap, cudaStream_t st)
 {

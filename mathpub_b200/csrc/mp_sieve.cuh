@@ -108,3 +108,5 @@ int mp_planes_run(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, TileSu
 // its primes go through the bucket scatter
 int mp_planes_geom(mp_handle *h, u64 lo, u64 hi, u32 block_log2, SieveGeom &g);
 int mp_planes_shape(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, u32 *tile_bits, u32 *bucket_above);
+// bytes of the buffers of a wave of that form, without what they may have to spare
+int mp_planes_bytes(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, u64 *bytes);
