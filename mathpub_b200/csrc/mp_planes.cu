@@ -73,7 +73,8 @@ __device__ __forceinline__ u32 plane_first(u64 is, u32 q, u32 m, const u16 *uv)
 }
 
 // (i0 + off) mod q from r = i0 mod q, which a launch of its own took once for the wave, and M = floor(2^32
-// / q): a 32-bit remainder instead of a 64-bit one.  r + off < 2^32: q < 2^21, off < 2^31
+// / q): a 32-bit remainder instead of a 64-bit one.  The quotient is at most 2 short, so 3 q and r + off have to be below 2^32,
+// which plan_planes sees to: off < 2^31, and q is a prime below the buckets (up to 1.5 tiles, 2654208, and a few primes more)
 __device__ __forceinline__ u32 plane_mod(u32 r, u32 off, u32 q, u32 M)
 {
     const u32 x = r + off;
@@ -1197,6 +1198,10 @@ static int plan_planes(mp_handle *h, const PrimeTable &tb, const SieveGeom &g, u
             P.cap = plane_bucket_cap(P.pt, tb.inv_prefix[P.iend] - tb.inv_prefix[P.it1], g.base / 30, tb.host[P.iend - 1]);
             // records of a wave within 3 GB
             if ((u64)P.cap * 8 * P.nb * 4 > (3072ull << 20) && P.tw > 1) continue;
+        }
+        if (P.it1 && ((u64)tb.host[P.it1 - 1] + (u64)P.nb * P.pt >> 32 || 3ull * tb.host[P.it1 - 1] >> 32)) {
+            if (P.tw > 1) continue;
+            return mp_set_error(h, MP_ERANGE, "a plane's wave is too long for 32-bit remainders");
         }
         MP_TRY(plan_sizes(h, P));
         if (P.psize + P.tsize + P.rsize > most && P.tw > 1) continue;
