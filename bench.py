@@ -155,12 +155,44 @@ def _odd_part(x):
 
 TD_PRIMES = [3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37, 41, 43, 47, 53, 59, 61, 67, 71, 73, 79, 83, 89, 97, 101, 103,
              107, 109, 113, 127]
-# 32-bit multiply or multiply-add instructions (the multiply pipe) in one Montgomery product:
-# two limbs, 8 for the product, 4 for m = t n^-1 mod 2^64 and 7 for the high half of m n (the
-# subtracting reduction, mp_mont64.cuh); three limbs of the Fermat kernel, three rows of
-# 3 + 3 (a b_i) + 1 (m) + 3 + 3 (m N) (mp_fermat.cu)
+# 32-bit multiply or multiply-add instructions (the multiply pipe; a 64-bit product is two) of the ladders' parts.
+# BPSW (mp_mont64.cuh): a two-limb product of the Lucas ladder, 8 for the product, 4 for m = t n^-1 mod 2^64 and 7
+# for the high half of m n; a squaring of the base-2 ladder, below 2^63 and above; one of its shifts, one word of
+# reduction.  Three-limb Fermat ladder (mp_fermat.cu): a squaring, a shift, leaving Montgomery form.
 IMAD_PER_PRODUCT_BPSW = 19
-IMAD_PER_PRODUCT_FERMAT_K3 = 39
+IMAD_PER_SQUARING_BASE2 = (16, 18)
+IMAD_PER_SHIFT_BASE2 = 5
+IMAD_PER_SQUARING_FERMAT_K3 = 33
+IMAD_PER_SHIFT_FERMAT_K3 = 7
+IMAD_LEAVE_FERMAT_K3 = 21
+
+
+def base2_multiplies(n):
+    """Multiply instructions of the base-2 ladders of odd n > 2 (an array), each: w digits of five bits below a top
+    of at most seven, w = (bitlen(n) - 4) / 5 or fewer while 2^(5 w) passes d (n - 1 = d 2^s); five squarings and a
+    shift a digit, and one more shift for each 32 that the top is above 63."""
+    n = np.asarray(n, dtype=np.uint64)
+    d = _odd_part(n - np.uint64(1))
+    w = np.where(_bitlen64(n) > 8, (_bitlen64(n).astype(np.int64) - 4) // 5, 0)
+    w = np.minimum(w, (_bitlen64(d).astype(np.int64) - 1) // 5)
+    top = (d >> (5 * w).astype(np.uint64)).astype(np.int64)
+    sq = np.where(n >> np.uint64(63) == 0, IMAD_PER_SQUARING_BASE2[0], IMAD_PER_SQUARING_BASE2[1])
+    return w * (5 * sq + IMAD_PER_SHIFT_BASE2) + -(-np.maximum(top - 63, 0) // 32) * IMAD_PER_SHIFT_BASE2
+
+
+def fermat_multiplies_k3(bits):
+    """Multiply instructions of the three-limb Fermat ladder for a p - 1 of that many bits: squarings below its top
+    six bits, a shift for each five of them and one for the rest, and the way out of Montgomery form."""
+    t = max(0, bits - 6)
+    return t * IMAD_PER_SQUARING_FERMAT_K3 + -(-t // 5) * IMAD_PER_SHIFT_FERMAT_K3 + IMAD_LEAVE_FERMAT_K3
+
+
+def trial_survivors(n):
+    n = np.asarray(n, dtype=np.uint64)
+    surv = ((n & np.uint64(1)) == 1) & (n >= np.uint64(131 * 131))
+    for q in TD_PRIMES:
+        surv &= (n % np.uint64(q)) != 0
+    return surv
 
 
 def bpsw_products(n, prime_mask):
@@ -171,9 +203,7 @@ def bpsw_products(n, prime_mask):
     mod 5, four otherwise).  The squarings of the strong chains after the ladders and the set-up
     are left out, so this is a lower bound on the work."""
     n = np.asarray(n, dtype=np.uint64)
-    surv = ((n & np.uint64(1)) == 1) & (n >= np.uint64(131 * 131))
-    for q in TD_PRIMES:
-        surv &= (n % np.uint64(q)) != 0
+    surv = trial_survivors(n)
     ns = n[surv]
     sprp = int((_bitlen64(_odd_part(ns - np.uint64(1))) - 1).sum())
     npr = n[surv & prime_mask]
@@ -347,6 +377,7 @@ def run_ours(args):
     bpsw_primes = int(np.unpackbits(bpsw_bits.view(np.uint8)).sum())
     pmask = np.unpackbits(bpsw_bits.view(np.uint8), bitorder="little")[:len(flat)].astype(bool)
     sprp_products, lucas_products, bpsw_survivors, bpsw_lucas_n = bpsw_products(flat, pmask)
+    base2_ops = int(base2_multiplies(flat[trial_survivors(flat)]).sum())
 
     peaks = e.probe_peaks()
     hbm, hbm_src = peaks_file()
@@ -445,16 +476,17 @@ def run_ours(args):
                      "plain_tests_per_s": world * BPSW_COUNT / (bpsw_plain_ms / 1e3),
                      "plain_ms_per_batch": bpsw_plain_ms, "batched_over_plain": bpsw_plain_ms / bpsw_ms,
                      "same_verdicts": bpsw_same, "primes": bpsw_primes,
-                     "roofline": imad_roofline((sprp_products + lucas_products) * IMAD_PER_PRODUCT_BPSW, bpsw_ms,
+                     "roofline": imad_roofline(base2_ops + lucas_products * IMAD_PER_PRODUCT_BPSW, bpsw_ms,
                                                peaks["imad32"], {
-                         "products_base2_ladders": sprp_products, "products_lucas_ladders": lucas_products,
+                         "exponent_bits_base2_ladders": sprp_products, "multiplies_base2_ladders": base2_ops,
+                         "products_lucas_ladders": lucas_products,
                          "candidates_past_trial_division": bpsw_survivors, "lucas_candidates": bpsw_lucas_n,
-                         "imad_per_product": IMAD_PER_PRODUCT_BPSW,
-                         "note": "achieved = Montgomery products counted exactly from the inputs (base-2 ladders of "
-                                 "the trial-division survivors, Lucas ladders of the primes; chain squarings and "
-                                 "set-up left out: a lower bound) x 32-bit multiply instructions per product / "
-                                 "kernel time; a squaring of the batched ladders takes fewer instructions than a "
-                                 "product, so frac can pass 1; peak = the 32-bit IMAD rate measured in this run"}),
+                         "imad_per_squaring_base2": list(IMAD_PER_SQUARING_BASE2),
+                         "imad_per_product_lucas": IMAD_PER_PRODUCT_BPSW,
+                         "note": "achieved = 32-bit multiply instructions of the ladders, counted exactly from the "
+                                 "inputs (base-2 ladders of the trial-division survivors: squarings and shifts; Lucas "
+                                 "ladders of the primes: products; chain squarings, set-up and trial division left "
+                                 "out: a lower bound) / kernel time; peak = the 32-bit IMAD rate measured in this run"}),
                      "workload": "2^26 seeded odd u64 (60% uniform [2^40,2^64), 30% p*q near 2^62, "
                                  "10% (k+1)(2k+1) / Chernick), 4096 lists, log-uniform lengths"},
             "config1": config1,
@@ -581,14 +613,12 @@ def run_fermat(e, world, rank, dev, imad_peak):
         fix = all(r[k] == c4[k] for k in ("primes", "tests", "near", "flt", "cks", "ordered_hash")) if lo == 10 ** 12 else None
     except Exception:
         pass
-    # products per prime: one per bit of p - 1 (square and double folded into one product where
-    # 8N < R) and the multiply that leaves Montgomery form; every p in the range has 40 bits
-    products = r["tests"] * (40 + 1)
-    roof = imad_roofline(products * IMAD_PER_PRODUCT_FERMAT_K3, kms, imad_peak, {
-        "products": products, "imad_per_product": IMAD_PER_PRODUCT_FERMAT_K3,
-        "note": "achieved = (bitlen(p - 1) + 1) three-limb Montgomery products per prime x 39 32-bit multiply "
-                "instructions per product / time of the quotient and statistics kernels; the ladder's squarings take "
-                "fewer and its first bits none, so frac can pass 1"})
+    # every p - 1 of the range has 40 bits: 34 squarings, 7 shifts and the way out of Montgomery form
+    per_prime = fermat_multiplies_k3(40)
+    roof = imad_roofline(r["tests"] * per_prime, kms, imad_peak, {
+        "imad_per_prime": per_prime, "imad_per_squaring": IMAD_PER_SQUARING_FERMAT_K3,
+        "note": "achieved = 32-bit multiply instructions of a prime's ladder (set-up, quotient and statistics left "
+                "out: a lower bound) x primes / time of the quotient and statistics kernels"})
     return {"workload": "base-2 Fermat quotients of every prime in [1e12, 1e12+4e9) (per rank), 3-limb Montgomery",
             "tests": r["tests"], "tests_per_s": r["tests"] / (kms / 1e3), "kernel_ms": kms, "roofline": roof,
             "e2e_tests_per_s": r["tests"] / wall, "e2e_ms": wall * 1e3, "near": r["near"], "flt": r["flt"],
