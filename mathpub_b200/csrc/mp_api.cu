@@ -377,7 +377,12 @@ int mp_fermat_q_base2(mp_handle *h, const uint64_t *p, size_t count, uint64_t *q
     std::lock_guard<std::recursive_mutex> lk(h->mu);
     MP_CUDA(h, cudaSetDevice(h->device));
     u64 any = 0;                                   // the bits that any p has
-    for (size_t i = 0; i < count; i++) any |= p[i];
+    // eight at a time: one by one the loop's time hung on where the code fell (2^20 quotients at 1e16: 1.94 or 2.02
+    // ms a call from one build to the next; 1.94 so)
+    size_t i = 0;
+    for (; i + 8 <= count; i += 8)
+        any |= ((p[i] | p[i + 1]) | (p[i + 2] | p[i + 3])) | ((p[i + 4] | p[i + 5]) | (p[i + 6] | p[i + 7]));
+    for (; i < count; i++) any |= p[i];
     if (any >> 63) return mp_set_error(h, MP_ERANGE, "p must be below 2^63");
     Prefault pages(q_out, count * 8);
     cudaStream_t st = h->stream;
