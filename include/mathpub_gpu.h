@@ -239,7 +239,7 @@ int mp_bpsw_batches(mp_handle *h, const uint64_t *const *lists, const uint32_t *
    multiple of 32, host array offs[0..nlists]), verdict words (u32, bit i & 31 of word
    i >> 5) at d_bits + offs[i] / 32; mode MP_MODE_BATCHED (launches over every list at
    once: trial division, the base-2 test on the survivors, Selfridge's search and the Lucas
-   test on the passers; one launch for a few thousand candidates) or MP_MODE_PLAIN (one launch per list) */
+   test on the passers; one launch for up to 16384 candidates) or MP_MODE_PLAIN (one launch per list) */
 int mp_bpsw_lists_dev(mp_handle *h, const uint64_t *d_n, const uint64_t *offs,
                       const uint32_t *lens, uint32_t nlists, uint32_t *d_bits, uint32_t mode,
                       void *stream);

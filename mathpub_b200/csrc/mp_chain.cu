@@ -244,20 +244,21 @@ __device__ __forceinline__ void cs_and_group(u32 (&acc)[4][4], const uint4 *__re
 
 // one CTA per CS_CPB classes of one segment: AND the rotated patterns over each class's 2^17
 // values of k and append the survivors' offsets from the unit's base.  The rotations of all
-// the CTA's classes and groups are taken in parallel before one barrier, and with them the number of k that a class has
-// up to the unit's last offset: compared in 32 bits, and only in classes that end before their last k.  (A
-// 64-bit product and comparison per chunk in every class: 5.2 instead of 4.4 ms for 1e13 integers at k = 11, 301 instead of
-// 272 for 1e15; without the test for dead chunks 4.9 and 443 with the smaller wheel.)  The windows' places take
-// as much shared memory as there are groups, and leave the rest to L1.
+// the CTA's classes and groups are taken in parallel before one barrier, and with them the number of
+// k that a class has up to the unit's last offset: compared in 32 bits, and only in classes that end
+// before their last k.  (A 64-bit product and comparison per chunk in every class: 5.2 instead of 4.4 ms
+// for 1e13 integers at k = 11, 301 instead of 272 for 1e15; without the test for chunks past the end 4.9
+// for 1e13.)  The windows' places take as much shared memory as there are groups, and leave the rest to L1.
 #define CS_CPB 8u                             // classes per CTA
 #define CS_CPT (CS_K / 128 / CS_THREADS)      // 128-bit chunks per thread and class
 static_assert(CS_CPT == 4, "cs_and_group takes 4 chunks per thread");
 __global__ void __launch_bounds__(CS_THREADS) cs_sieve_kernel(CsTables T, CsShape S, CsUnit U, u64 *list, u64 cap,
                                                               ull *count)
 {
-    extern __shared__ __align__(8) u32 s_win[];   // of class c and group gi, at 2 (c ngroups + gi): the first 16-byte chunk
-                                                  // of the window, its bit offset in that chunk
-    __shared__ u32 s_s0[CS_CPB], s_room[CS_CPB];   // per class: first offset, values of k up to the unit's last offset
+    // of class c and group gi, at 2 (c ngroups + gi): the first 16-byte chunk of the window, its bit offset in
+    // that chunk
+    extern __shared__ __align__(8) u32 s_win[];
+    __shared__ u32 s_s0[CS_CPB], s_room[CS_CPB];  // per class: first offset, values of k up to the unit's last offset
     const u32 nblk = (U.nj + CS_CPB - 1) / CS_CPB;
     const u32 jb = blockIdx.x % nblk, g = blockIdx.x / nblk;
     const u32 *bq = U.bq + (size_t)g * T.nps;
@@ -511,7 +512,8 @@ static void cs_queue_unit(const CsTables &T, const CsShape &S, const CsUnit &U, 
 {
     const u32 rounds = std::min(split, S.k);
     cudaMemsetAsync(L.cnt, 0, (size_t)(rounds + 2) * sizeof(ull), st);
-    cs_sieve_kernel<<<(U.nj + CS_CPB - 1) / CS_CPB * U.nseg, CS_THREADS, CS_CPB * T.ngroups * 8, st>>>(T, S, U, L.list[0], L.cap, L.cnt);
+    cs_sieve_kernel<<<(U.nj + CS_CPB - 1) / CS_CPB * U.nseg, CS_THREADS, CS_CPB * T.ngroups * 8, st>>>(
+        T, S, U, L.list[0], L.cap, L.cnt);
     const unsigned grid = (unsigned)sm_count * 8;
     int cur = 0;
     for (u32 r = 0; r < rounds; r++, cur ^= 1)

@@ -73,8 +73,9 @@ __device__ __forceinline__ u32 plane_first(u64 is, u32 q, u32 m, const u16 *uv)
 }
 
 // (i0 + off) mod q from r = i0 mod q, which a launch of its own took once for the wave, and M = floor(2^32
-// / q): a 32-bit remainder instead of a 64-bit one.  The quotient is at most 2 short, so 3 q and r + off have to be below 2^32,
-// which plan_planes sees to: off < 2^31, and q is a prime below the buckets (up to 1.5 tiles, 2654208, and a few primes more)
+// / q): a 32-bit remainder instead of a 64-bit one.  The quotient is at most 2 short, so 3 q and r + off have to
+// be below 2^32, which plan_planes sees to: off < 2^31, and q is a prime below the buckets (up to 1.5 tiles,
+// 2654208, and a few primes more)
 __device__ __forceinline__ u32 plane_mod(u32 r, u32 off, u32 q, u32 M)
 {
     const u32 x = r + off;
@@ -709,8 +710,8 @@ __device__ __forceinline__ u32 run_starts(u32 any, u32 next, bool prev, u32 Z)
 // between 30 z + 2 and 30 z + 58, so once a gap of g is known only runs of at least (g - 28) / 30
 // empty blocks can hold a wider one, and of at least (g - 30) / 30 one as wide, which are rare.  A gap as
 // wide counts where it may come first: against another warp's, and in the row whose own search for long
-// runs first gave g, since the earliest of equal gaps can have a block fewer than the one found.  Until (g - 30) / 30 is at
-// least 1 the row's primes are walked.
+// runs first gave g, since the earliest of equal gaps can have a block fewer than the one found.  Until
+// (g - 30) / 30 is at least 1 the row's primes are walked.
 // 0.43 ms for 2^33 integers without the bitmap (4.6 GB of planes a ms: issue and the latency of a row),
 // 0.6 in the odd-only tiles; a short range waits some 20 us for one stretch's rows
 template <bool BITMAP>

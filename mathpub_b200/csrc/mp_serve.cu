@@ -15,8 +15,8 @@
 //                      prime that starts it (each chunk sees the primes past its end);
 //                      K workers overlap on the device;
 //   primality request  a worker that picks one takes every primality request waiting at
-//                      that moment (up to a candidate cap) and runs them as ONE persistent
-//                      batched BPSW launch over all their lists (continuous batching).
+//                      that moment (up to a candidate cap) and runs them as ONE batched BPSW
+//                      call over all their lists (continuous batching).
 // Results are those of the same request run alone: the kernels are the same and every
 // request has its own outputs; only scheduling differs.
 #include "mp_common.cuh"
