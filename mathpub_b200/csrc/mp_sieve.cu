@@ -2074,7 +2074,7 @@ static int pick_geometry(mp_handle *h, const mp_sieve_opts *o, u32 &tlog, int &n
 
 // whether a batched call runs in residue planes (mp_planes.cu): unless the call or the handle pins a
 // geometry or form of the odd-only tiles.  Measured from 2^16 to 2^30 integers, with and without hashes, as a call:
-// against the tiles of 2^20 bits, which unpinned calls took before, 0.92 of the time at the most (2^28 at 1e12) and
+// against the tiles of 2^20 bits, which unpinned calls took before, the same time at the most (2^28 at 1e9) and
 // 0.3 at the least (2^26 at 9e17); against the best of the smaller tiles, which a call may pin, 1.28 to 0.98 times at 1e9 up
 // to 2^27, where few primes sieve (2^26: 92 us, 72 in tiles of 2^18 bits), 1.01 to 0.6 times at 1e12 and less above.
 static bool planes_form(const mp_handle *h, const mp_sieve_opts *o)
